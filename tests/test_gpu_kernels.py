@@ -171,6 +171,32 @@ def test_many_tokens_in_float32_take_the_large_tiles_and_keep_the_order_of_the_s
     assert torch.equal(other, plain)
 
 
+@pytest.mark.parametrize("N,K_", [(65, 1024), (130, 1028), (64, 2052), (3, 8196), (200, 14336)])
+def test_float32_sums_in_segments_of_k(K, N, K_):
+    """Float operands: the K range is cut into at most eight segments whose sums are added in order, by the blocks of a
+    cluster where rows start on 16-byte boundaries and by one block where they do not.  Every number of tokens (the
+    kernels' tiles take up to 1, 2, 4, 8, 16, 32, 64, then 64 or 128 at a time) gives the same bits, and the sums lie
+    within the bound of their own order of additions: the products of a segment one after another, then the segments."""
+    n = min(8, -(-K_ // 1024))
+    seg = -(-(-(-K_ // n)) // 128) * 128
+    x, w = rnd((200, K_), torch.float32, seed=21).to(DEV), rnd((N, K_), torch.float32, seed=22).to(DEV)
+    b = rnd((N,), torch.float32, seed=23).to(DEV)
+    out = torch.full((200, N), 9.0, device=DEV)
+    K.gemm_generic(x, w, out, bias=b)
+    want = x.double() @ w.double().t() + b.double()
+    bound = (min(seg, K_) + n + 1) * 2.0 ** -24 * (x.abs().double() @ w.abs().double().t() + b.abs().double())
+    assert ((out.double() - want).abs() <= bound).all()
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129, 192):
+        part = torch.full((M, N), 9.0, device=DEV)
+        K.gemm_generic(x[:M], w, part, bias=b)
+        assert torch.equal(part, out[:M]), M
+    odd = torch.zeros(200, K_ + 4, device=DEV)
+    odd[:, 1:1 + K_] = x
+    part = torch.empty(200, N, device=DEV)
+    K.gemm_generic(odd[:, 1:1 + K_], w, part, bias=b)
+    assert torch.equal(part, out)
+
+
 def test_gemm_generic_strided_rows_and_true_float32(K):
     """Rows of a wider buffer; and float32 products are not rounded to a shorter mantissa."""
     buf = rnd((10, 100), torch.float32, seed=9).to(DEV)
