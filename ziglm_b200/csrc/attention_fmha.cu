@@ -10,15 +10,21 @@
 // swizzle; a K stage is free as soon as the scores are computed, a V stage after P V); warp 1 issues
 // the tcgen05.mma instructions (K pages are K-major operands, V pages MN-major ones, both exactly as
 // the cache stores them) in the order  P_0 V, S_0 of the next step, P_1 V, S_1 of the next step, so
-// that the tensor core works for one tile while the softmax of the other runs; warps 2-5 are the
-// softmax of tile 0 and warps 6-9 of tile 1: thread r owns query row r, reads its row of S with
+// that the tensor core works for one tile while the softmax of the other runs; warps 4-7 are the
+// softmax of tile 0 and warps 8-11 of tile 1 (warps 2 and 3 complete the first warpgroup, which gives
+// registers to the others): thread r owns query row r, reads its row of S with
 // tcgen05.ld (all 128 scores issued together and waited for once; the row stays in registers between
 // the maximum and the exponentials), keeps the running maximum and sum in float (base 2, scale folded
-// in), writes the probabilities with tcgen05.st, and rescales O in tensor memory when its maximum has moved by more
+// in), writes the probabilities with tcgen05.st a page at a time (P V of the first page runs under the
+// exponentials of the second), and rescales O in tensor memory when its maximum has moved by more
 // than 2^8 (a rescale that is skipped leaves probabilities up to 256, well inside bf16 and float
 // range, and cancels in O / l).  The tensor core runs its instructions in the order of issue, so when
 // S_t of a step is there, P_t V of the step before is complete: the softmax may touch O_t and
 // overwrite the old probabilities without another wait.
+// What bounds it: a step of both tiles takes about 3,900 clocks, 2,048 of the tensor core and 2,048 of the
+// exponentials' unit, which a tile alternates between (softmax 1,900, products and hand-over 1,900).  One sequence of
+// 16,001 tokens, 32 heads of 128: 2.62 -> 1.91 ms (1,100 TFLOP/s), of 2,048 tokens 65 -> 52 us, 64 sequences of 18 to
+// 1,008 tokens with 32 heads of 64: 573 -> 465 us, nearly all of it the issuing warp's (see there).
 // The formulas are those of attention.cu (the reference's src/model.zig:659-700): scores scaled
 // after the dot product, keys [start, pos] visible, softmax with maximum subtraction, weighted sum.
 // Every mbarrier wait is bounded and reports through an error word.
@@ -37,7 +43,11 @@ constexpr int FM_ROWS = FM_BQ * FM_TILES;
 constexpr int FM_PAGE = 64;          // keys per page
 constexpr int FM_NP = 2;             // pages per step
 constexpr int FM_KEYS = FM_PAGE * FM_NP;
-constexpr int FM_THREADS = 320;      // TMA warp, MMA warp, four softmax warps per tile
+constexpr int FM_THREADS = 384;      // a warpgroup with the TMA warp and the MMA warp, then one of softmax warps per tile
+// Registers a thread after the split: what the block was launched with (168 x 384) is shared out again, so that a
+// softmax thread keeps its row of 128 scores in registers (with 168 it spilled some of them every step).
+constexpr int FM_REGS_ISSUE = 88, FM_REGS_SOFTMAX = 208;
+static_assert(FM_REGS_ISSUE + 2 * FM_REGS_SOFTMAX <= 3 * 168, "the shares must fit what the block was launched with");
 constexpr int ERR_FM_ALIGN = 20, ERR_FM_Q = 21, ERR_FM_KV = 22, ERR_FM_S = 23, ERR_FM_P = 24, ERR_FM_O = 25, ERR_FM_EMPTY = 26;
 
 template <int HD> struct FmCfg {
@@ -61,6 +71,28 @@ __device__ __forceinline__ bool warp_mbar_wait(uint32_t bar, uint32_t parity, vo
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
+template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// Two floats at once (the same roundings as one by one, half the instructions), and the larger of three.
+__device__ __forceinline__ void fma_pair(uint32_t& x, uint32_t& y, unsigned long long b, unsigned long long c) {
+    asm("{\n\t.reg .b64 t;\n\tmov.b64 t, {%0, %1};\n\tfma.rn.f32x2 t, t, %2, %3;\n\tmov.b64 {%0, %1}, t;\n\t}"
+        : "+r"(x), "+r"(y) : "l"(b), "l"(c));
+}
+__device__ __forceinline__ void add_pair(unsigned long long& sum, uint32_t x, uint32_t y) {
+    asm("{\n\t.reg .b64 t;\n\tmov.b64 t, {%1, %2};\n\tadd.rn.f32x2 %0, %0, t;\n\t}" : "+l"(sum) : "r"(x), "r"(y));
+}
+__device__ __forceinline__ unsigned long long pair_of(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(__float_as_uint(x)), "r"(__float_as_uint(y)));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
 struct FmArgs {
     __nv_bfloat16* out;
     int n_heads, n_kv;
@@ -79,11 +111,13 @@ struct FmArgs {
 };
 
 // The softmax of one query row over a step of NP pages: S from tensor memory, P (bf16) back over its first
-// half.  Returns the factor by which the running sum was rescaled; updates m (reference maximum, base 2) and l.
+// half, page after page; p_bar (one barrier a page) hears of every page as soon as its probabilities are written, so
+// that the product with its values runs while the next page's exponentials are taken.  Updates m (reference maximum,
+// base 2) and l.
 template <int HD, int NP, bool SLOPES>
-__device__ __forceinline__ float softmax_row(uint32_t t_s, uint32_t t_o, bool full, int lo_vis, int hi_vis, int keep_vis,
-                                             float scale, float neg_big, int lt, float& m, float& l, float cap_in2,
-                                             float cap_log2, float slope, float bias0) {
+__device__ __forceinline__ void softmax_row(uint32_t t_s, uint32_t t_o, bool full, int lo_vis, int hi_vis, int keep_vis,
+                                            float scale, float neg_big, int lt, float& m, float& l, float cap_in2,
+                                            float cap_log2, float slope, float bias0, uint32_t p_bar, int lane) {
     constexpr int N = NP * FM_PAGE;
     uint32_t v[N];
 #pragma unroll
@@ -109,21 +143,17 @@ __device__ __forceinline__ float softmax_row(uint32_t t_s, uint32_t t_o, bool fu
             v[i] = __float_as_uint(fmaf(__uint_as_float(v[i]), scale, fmaf((float)i, slope, bias0)));
         scale = 1.0f;
     }
-    float mx8[8];
+    if (!full) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) mx8[i] = neg_big;
-    if (full) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) mx8[i & 7] = fmaxf(mx8[i & 7], __uint_as_float(v[i]));
-    } else {
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
+        for (int i = 0; i < N; ++i)
             if ((i < lo_vis && i >= keep_vis) || i > hi_vis) v[i] = __float_as_uint(neg_big);   // stays masked below
-            mx8[i & 7] = fmaxf(mx8[i & 7], __uint_as_float(v[i]));
-        }
     }
-    const float mx_raw = fmaxf(fmaxf(fmaxf(mx8[0], mx8[1]), fmaxf(mx8[2], mx8[3])),
-                               fmaxf(fmaxf(mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7])));
+    float mx4[4] = {neg_big, neg_big, neg_big, neg_big};
+#pragma unroll
+    for (int i = 0; i < N; i += 8)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mx4[j] = max3(mx4[j], __uint_as_float(v[i + 2 * j]), __uint_as_float(v[i + 2 * j + 1]));
+    const float mx_raw = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
     const float mx = mx_raw == neg_big ? -INFINITY : mx_raw * scale;       // the scale is positive
     // the reference maximum moves only when the true one has grown by more than 8 (in base 2)
     float corr = 1.0f;
@@ -135,38 +165,50 @@ __device__ __forceinline__ float softmax_row(uint32_t t_s, uint32_t t_o, bool fu
     // rescale O when some row of the warp moved its reference (never in the first step: O is empty)
     if (lt > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
 #pragma unroll 1
-        for (int c = 0; c < HD / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld32(t_o + c * 32, o);
+        for (int c = 0; c < HD / 16; ++c) {
+            uint32_t o[16];
+            tmem_ld16(t_o + c * 16, o);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
-            tmem_st32(t_o + c * 32, o);
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+            tmem_st16(t_o + c * 16, o);
         }
     }
-    // stage by stage over the row: neighbouring instructions never depend on one another
-    float sum8[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) sum8[i] = 0.f;
+    // stage by stage over 32 scores: neighbouring instructions never depend on one another
+    const unsigned long long scale2 = pair_of(scale, scale), use2 = pair_of(-use, -use);
+    unsigned long long sum2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
     for (int c = 0; c < N / 32; ++c) {
-        float x[32];
+        uint32_t* x = &v[c * 32];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) x[i] = fmaf(__uint_as_float(v[c * 32 + i]), scale, -use);   // masked: about -3e38
+        for (int i = 0; i < 32; i += 2) fma_pair(x[i], x[i + 1], scale2, use2);                 // masked: about -3e38
 #pragma unroll
-        for (int i = 0; i < 32; ++i) asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(x[i]) : "f"(x[i]));
+        for (int i = 0; i < 32; ++i)
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=r"(x[i]) : "r"(x[i]));
 #pragma unroll
-        for (int i = 0; i < 32; ++i) sum8[i & 7] += x[i];
+        for (int i = 0; i < 32; i += 2) add_pair(sum2[(i >> 1) & 3], x[i], x[i + 1]);
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            __nv_bfloat162 pp = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+            __nv_bfloat162 pp = __floats2bfloat162_rn(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1]));
             pk[i] = *reinterpret_cast<uint32_t*>(&pp);
         }
         tmem_st16(t_s + c * 16, pk);
+        if (c & 1) {                                            // a page of 64 keys is written
+            tmem_st_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(p_bar + 8 * (c >> 1));
+                if (NP == 1) mbar_arrive(p_bar + 8);            // the other page's barrier keeps its count of steps
+            }
+        }
     }
-    l = l * corr + (((sum8[0] + sum8[1]) + (sum8[2] + sum8[3])) + ((sum8[4] + sum8[5]) + (sum8[6] + sum8[7])));
-    return corr;
+    float s8[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(s8[2 * i]), "=f"(s8[2 * i + 1]) : "l"(sum2[i]));
+    l = l * corr + (((s8[0] + s8[1]) + (s8[2] + s8[3])) + ((s8[4] + s8[5]) + (s8[6] + s8[7])));
 }
 
 template <int HD, bool SLOPES>
@@ -190,12 +232,12 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const uint32_t k_full0 = bar + 8, k_empty0 = k_full0 + 8 * C::NK;
     const uint32_t v_full0 = k_empty0 + 8 * C::NK, v_empty0 = v_full0 + 8 * C::NV;
     const uint32_t s_full0 = v_empty0 + 8 * C::NV;                   // [tile]: the scores of a step are there
-    const uint32_t p_full0 = s_full0 + 8 * FM_TILES;                 // [tile]: the probabilities are written
-    const uint32_t o_full0 = p_full0 + 8 * FM_TILES;                 // [tile]: the last P V is complete
+    const uint32_t p_full0 = s_full0 + 8 * FM_TILES;                 // [tile][page]: the probabilities are written
+    const uint32_t o_full0 = p_full0 + 8 * FM_TILES * FM_NP;         // [tile]: the last P V is complete
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem + (o_full0 + 8 * FM_TILES - base));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int b = blockIdx.y, h = blockIdx.x;
     const int tok_begin = a.cu_seqlens[b], n_new = a.cu_seqlens[b + 1] - tok_begin;
     // The last query tiles see the most keys.  Blocks start in the order of their indices (x fastest), so the
@@ -257,7 +299,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         for (int s = 0; s < C::NV; ++s) { mbar_init(v_full0 + 8 * s, 1); mbar_init(v_empty0 + 8 * s, 1); }
         for (int t = 0; t < FM_TILES; ++t) {
             mbar_init(s_full0 + 8 * t, 1);
-            mbar_init(p_full0 + 8 * t, 4);       // one arrival per softmax warp of the tile
+            for (int pg = 0; pg < FM_NP; ++pg) mbar_init(p_full0 + 8 * (t * FM_NP + pg), 4);   // one arrival per softmax warp of the tile
             mbar_init(o_full0 + 8 * t, 1);
         }
         *abort_flag = 0;
@@ -273,6 +315,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const uint32_t tmem_base = *tmem_holder;
     pdl_launch_dependents();
     pdl_wait();                       // queries, keys and values of this step are written by earlier kernels
+    if (warp < 4) regs_dec<FM_REGS_ISSUE>();      // this warpgroup gives registers to the two of softmax warps
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -334,67 +377,71 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc_s2 = idesc_bf16(FM_BQ, FM_KEYS);         // S: 128 x 128 keys, K = head_dim
-            constexpr uint32_t idesc_s1 = idesc_bf16(FM_BQ, FM_PAGE);         // a last step of one page
-            constexpr uint32_t idesc_o = idesc_bf16_b_mn(FM_BQ, HD);          // O: 128 x head_dim, K = 16 keys
-            bool alive = mbar_wait(q_full, 0, abort_flag, a.err, ERR_FM_Q);
-            // step j: for each tile first P V of step j - 1, then the scores of step j
-            for (int j = 0; j <= n_steps && alive; ++j) {
+        // The warp walks the steps together and one elected lane issues: descriptors and addresses are then the same
+        // in every lane, and the compiler keeps them in the registers the instructions take them from.  (Inside a
+        // branch of one lane every instruction cost 80 to 200 clocks to issue, more than the 64 it runs.)
+        constexpr uint32_t idesc_s2 = idesc_bf16(FM_BQ, FM_KEYS);         // S: 128 x 128 keys, K = head_dim
+        constexpr uint32_t idesc_s1 = idesc_bf16(FM_BQ, FM_PAGE);         // a last step of one page
+        constexpr uint32_t idesc_o = idesc_bf16_b_mn(FM_BQ, HD);          // O: 128 x head_dim, K = 16 keys
+        const uint64_t dq = smem_desc_sw128(q_smem), dk = smem_desc_sw128(k_smem);
+        const uint64_t dv = smem_desc_sw128_mn(v_smem, FM_PAGE * 128);
+        bool alive = mbar_wait(q_full, 0, abort_flag, a.err, ERR_FM_Q);
+        // step j: for each tile first P V of step j - 1, then the scores of step j
+        for (int j = 0; j <= n_steps && alive; ++j) {
 #pragma unroll
-                for (int t = 0; t < FM_TILES; ++t) {
-                    if (!alive) break;
-                    const int jj = j - 1;
-                    if (runs(t, jj)) {
-                        const int sv = jj % C::NV, lt = local_step(t, jj);
-                        if (!mbar_wait(v_full0 + 8 * sv, (jj / C::NV) & 1, abort_flag, a.err, ERR_FM_KV) ||
-                            !mbar_wait(p_full0 + 8 * t, lt & 1, abort_flag, a.err, ERR_FM_P)) {
-                            alive = false;
-                            break;
-                        }
-                        tc_fence_after_sync();
-                        const int np = pages_of(jj);
-                        const uint32_t tmem_o = tmem_base + C::O_COL + t * HD;
-                        const uint32_t tmem_p = tmem_base + C::S_COL + t * FM_KEYS;
-                        for (int pg = 0; pg < np; ++pg) {
+            for (int t = 0; t < FM_TILES; ++t) {
+                const int jj = j - 1;
+                if (alive && runs(t, jj)) {
+                    const int sv = jj % C::NV, lt = local_step(t, jj);
+                    const int np = pages_of(jj);
+                    const uint32_t tmem_o = tmem_base + C::O_COL + t * HD;
+                    const uint32_t tmem_p = tmem_base + C::S_COL + t * FM_KEYS;
+                    alive = mbar_wait(v_full0 + 8 * sv, (jj / C::NV) & 1, abort_flag, a.err, ERR_FM_KV);
 #pragma unroll
-                            for (int ks = 0; ks < FM_PAGE / 16; ++ks) {
-                                const uint64_t db = smem_desc_sw128_mn(
-                                    v_smem + sv * C::KV_BYTES + pg * C::PAGE_BYTES + ks * 2048, FM_PAGE * 128);
-                                umma_bf16_ts(tmem_o, tmem_p + pg * (FM_PAGE / 2) + ks * 8, db, idesc_o,
-                                             (lt | pg | ks) != 0 ? 1u : 0u);
+                    for (int pg = 0; pg < FM_NP; ++pg) {
+                        if (pg < np) {
+                            alive = alive && mbar_wait(p_full0 + 8 * (t * FM_NP + pg), lt & 1, abort_flag, a.err, ERR_FM_P);
+                            alive = __all_sync(0xffffffffu, alive);
+                            tc_fence_after_sync();
+                            if (alive && elect_one()) {
+#pragma unroll
+                                for (int ks = 0; ks < FM_PAGE / 16; ++ks)
+                                    umma_bf16_ts(tmem_o, tmem_p + pg * (FM_PAGE / 2) + ks * 8,
+                                                 dv + (uint64_t)((sv * C::KV_BYTES + pg * C::PAGE_BYTES + ks * 2048) >> 4), idesc_o,
+                                                 (lt | pg | ks) != 0 ? 1u : 0u);
                             }
                         }
-                        if (jj == step_hi[t] - 1) umma_commit(o_full0 + 8 * t);
                     }
-                    if (j < n_steps && runs(t, j)) {
-                        const int sk = j % C::NK;
-                        if (!mbar_wait(k_full0 + 8 * sk, (j / C::NK) & 1, abort_flag, a.err, ERR_FM_KV)) {
-                            alive = false;
-                            break;
-                        }
-                        tc_fence_after_sync();
-                        const uint32_t tmem_s = tmem_base + C::S_COL + t * FM_KEYS;
-                        const uint32_t idesc_s = pages_of(j) >= FM_NP ? idesc_s2 : idesc_s1;
+                    if (alive && jj == step_hi[t] - 1 && elect_one()) umma_commit(o_full0 + 8 * t);
+                }
+                if (alive && j < n_steps && runs(t, j)) {
+                    const int sk = j % C::NK;
+                    alive = mbar_wait(k_full0 + 8 * sk, (j / C::NK) & 1, abort_flag, a.err, ERR_FM_KV);
+                    alive = __all_sync(0xffffffffu, alive);
+                    tc_fence_after_sync();
+                    const uint32_t tmem_s = tmem_base + C::S_COL + t * FM_KEYS;
+                    const uint32_t idesc_s = pages_of(j) >= FM_NP ? idesc_s2 : idesc_s1;
+                    if (alive && elect_one()) {
 #pragma unroll
-                        for (int ks = 0; ks < HD / 16; ++ks) {
-                            const uint64_t da = smem_desc_sw128(q_smem + t * C::Q_BYTES + (ks >> 2) * (FM_BQ * 128) + (ks & 3) * 32);
-                            const uint64_t db = smem_desc_sw128(k_smem + sk * C::KV_BYTES + (ks >> 2) * (FM_KEYS * 128) + (ks & 3) * 32);
-                            umma_bf16(tmem_s, da, db, idesc_s, ks != 0 ? 1u : 0u);
-                        }
+                        for (int ks = 0; ks < HD / 16; ++ks)
+                            umma_bf16(tmem_s, dq + (uint64_t)((t * C::Q_BYTES + (ks >> 2) * (FM_BQ * 128) + (ks & 3) * 32) >> 4),
+                                      dk + (uint64_t)((sk * C::KV_BYTES + (ks >> 2) * (FM_KEYS * 128) + (ks & 3) * 32) >> 4), idesc_s,
+                                      ks != 0 ? 1u : 0u);
                         umma_commit(s_full0 + 8 * t);
                     }
                 }
-                if (!alive) break;
-                // both tiles have issued what they read of these stages
+            }
+            // both tiles have issued what they read of these stages
+            if (alive && elect_one()) {
                 if (j >= 1) umma_commit(v_empty0 + 8 * ((j - 1) % C::NV));
                 if (j < n_steps) umma_commit(k_empty0 + 8 * (j % C::NK));
             }
         }
         __syncwarp();
-    } else {
+    } else if (warp >= 4) {
         // ---------------------------------------------------------------- softmax
-        const int t = (warp - 2) >> 2;                                // tile of this warp
+        regs_inc<FM_REGS_SOFTMAX>();
+        const int t = (warp - 4) >> 2;                                // tile of this warp
         const int q = warp & 3;                                       // TMEM lane quarter this warp may touch
         const int r = q * 32 + lane;                                  // query row of this thread within the tile
         const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
@@ -428,19 +475,14 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             // One reading of the row: the loads of all its scores are issued together and waited for once
             // (a tcgen05.ld and its wait cost about as much as the arithmetic on 32 scores), the row stays in
             // registers between the maximum and the exponentials, and the stores of P are waited for once.
-            float corr;
             const float bias0 = slope * (float)(key0 - pos);
+            const uint32_t p_bar = p_full0 + 8 * FM_NP * t;
             if (np == FM_NP)
-                corr = softmax_row<HD, FM_NP, SLOPES>(t_s, t_o, full, lo_vis, hi_vis, keep_vis, scale, neg_big, lt, m, l, a.cap_in2, a.cap_log2,
-                                              slope, bias0);
+                softmax_row<HD, FM_NP, SLOPES>(t_s, t_o, full, lo_vis, hi_vis, keep_vis, scale, neg_big, lt, m, l, a.cap_in2,
+                                               a.cap_log2, slope, bias0, p_bar, lane);
             else
-                corr = softmax_row<HD, 1, SLOPES>(t_s, t_o, full, lo_vis, hi_vis, keep_vis, scale, neg_big, lt, m, l, a.cap_in2, a.cap_log2,
-                                              slope, bias0);
-            (void)corr;
-            tmem_st_wait();
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(p_full0 + 8 * t);
+                softmax_row<HD, 1, SLOPES>(t_s, t_o, full, lo_vis, hi_vis, keep_vis, scale, neg_big, lt, m, l, a.cap_in2,
+                                           a.cap_log2, slope, bias0, p_bar, lane);
         }
         // O holds every step: normalise and store this thread's row
         if (alive && step_hi[t] > step_lo[t])
