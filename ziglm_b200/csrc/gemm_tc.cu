@@ -85,20 +85,29 @@ struct TcArgs {
 // Tokens staged per TMA store: the box height of the output's tensor map.
 __host__ __device__ constexpr int sub_rows(int bn) { return (bn == 16 || bn == 64) ? 16 : 32; }
 
+// DEEP: 0 the usual number of stages, n > 0 n stages; SPLIT_K + n: n stages and no staging area, for launches that
+// split K (their sums meet in the stages' memory).
+constexpr int SPLIT_K = 100;
+
 template <int BN, int DEEP = 0> struct TcCfg {
     // Narrow tiles (decode steps) keep few stages, so that three or four blocks fit an SM: the blocks of
     // the next product become resident while this one drains and request their weight tiles early.
     // DEEP: the gated product of a decode step runs as one tile of a megabyte of weights per block, at
     // most two blocks per SM; what bounds it is the bytes each block has in flight, so it takes a fourth
     // stage (measured: five and more cost the next product its early residence).
-    static constexpr int STAGES = BN <= 32 ? (DEEP ? DEEP : 3) : (BN == 128 ? 5 : 4);
+    // A product whose K is split takes four stages in the same room (no staging area), and five or six where there is at
+    // most one block an SM and more K blocks than four: a small product's weights (four K blocks a block) are then all
+    // requested before the kernel before it ends, and a lone block has enough bytes in flight for its SM's share of
+    // the memory's bandwidth.
+    static constexpr bool SPLIT = DEEP >= SPLIT_K;
+    static constexpr int STAGES = SPLIT ? DEEP - SPLIT_K : BN <= 32 ? (DEEP ? DEEP : 3) : (BN == 128 ? 5 : 4);
     static constexpr int B_BYTES = BN * TC_BK * 2;
     static constexpr int ACC_COLS = BN;                            // columns of one accumulator
     static constexpr int COLS = 2 * BN < 32 ? 32 : 2 * BN;         // two accumulators: a power of two >= 32
     static constexpr int SUB = sub_rows(BN);                       // tokens staged per TMA store
     static constexpr int NBUF = BN >= 128 ? 2 : 1;                 // staging buffers: a store drains while the next fills
     static constexpr int SUB_BYTES = SUB * TC_BM * 4;
-    static constexpr int STAGING = NBUF * SUB_BYTES;
+    static constexpr int STAGING = SPLIT ? 0 : NBUF * SUB_BYTES;
     static constexpr int SMEM = 1024 + STAGES * (A_BYTES + B_BYTES) + STAGING + 256;
 };
 
@@ -230,7 +239,7 @@ __device__ __forceinline__ void store_tile(const TcArgs& a, const CUtensorMap* t
 // Persistent: block b works on tiles b, b + gridDim.x, ...  The accumulator in tensor memory is
 // double-buffered, so the epilogue of one tile runs while the next tile's products are issued.
 template <int BN, int MODE, int DEEP>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(TC_THREADS, BN <= 32 ? 3 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                const __grid_constant__ CUtensorMap tmap_y, TcArgs a) {
     using C = TcCfg<BN, DEEP>;
@@ -254,8 +263,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 
     __shared__ float inv_s[64];                     // row scales of a product that completes a norm
     __shared__ float norm_red[2][4][4];             // sums of squares: [epilogue half][token of a group][warp]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = a.splits > 1 ? cluster_rank() : 0u;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    constexpr bool MAY_SPLIT = C::SPLIT || BN > 32;  // narrow tiles have a form of their own for split launches
+    const bool split = MAY_SPLIT && a.splits > 1;
+    const uint32_t rank = split ? cluster_rank() : 0u;
     const int kb0 = (int)rank * a.kb_per_split;
     int n_kb = a.kb_total - kb0;
     if (n_kb > a.kb_per_split) n_kb = a.kb_per_split;
@@ -336,32 +347,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        // the whole warp walks the stages, an elected lane issues (see gemm_pair_kernel)
+        {
             constexpr uint32_t idesc = idesc_bf16(TC_BM, BN);
-            int it = 0, local = 0;
+            const uint64_t da0 = smem_desc_sw128(a_base), db0 = smem_desc_sw128(b_base);
+            int s = 0, local = 0;
+            uint32_t parity = 0;
             bool alive = true;
             for (int tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x, ++local) {
                 const int ab = local & 1;
                 // the epilogue must have emptied this accumulator (two tiles ago)
-                if (!mbar_wait(acc_empty0 + 8 * ab, ((local >> 1) & 1) ^ 1u, abort_flag, a.err, ERR_WAIT_ACCUM)) break;
+                alive = __all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * ab, ((local >> 1) & 1) ^ 1u, abort_flag, a.err, ERR_WAIT_ACCUM));
+                if (!alive) break;
                 tc_fence_after_sync();
                 const uint32_t tmem_d = tmem_base + ab * C::ACC_COLS;
-                for (int kb = 0; kb < n_kb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait(full0 + 8 * s, (it / STAGES) & 1, abort_flag, a.err, ERR_WAIT_FULL)) {
-                        alive = false;
-                        break;
-                    }
+                for (int kb = 0; kb < n_kb; ++kb) {
+                    alive = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, parity, abort_flag, a.err, ERR_WAIT_FULL));
+                    if (!alive) break;
                     tc_fence_after_sync();
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < TC_BK / TC_UMMA_K; ++k) {
-                        const uint64_t da = smem_desc_sw128(a_base + s * A_BYTES + k * TC_UMMA_K * 2);
-                        const uint64_t db = smem_desc_sw128(b_base + s * C::B_BYTES + k * TC_UMMA_K * 2);
-                        umma_bf16(tmem_d, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
+                        for (int k = 0; k < TC_BK / TC_UMMA_K; ++k)
+                            umma_bf16(tmem_d, da0 + (uint64_t)((s * A_BYTES + k * TC_UMMA_K * 2) >> 4),
+                                      db0 + (uint64_t)((s * C::B_BYTES + k * TC_UMMA_K * 2) >> 4), idesc, (kb | k) != 0 ? 1u : 0u);
+                        umma_commit(empty0 + 8 * s);
                     }
-                    umma_commit(empty0 + 8 * s);
+                    if (++s == STAGES) { s = 0; parity ^= 1u; }
                 }
-                umma_commit(acc_full0 + 8 * ab);
+                if (elect_one()) umma_commit(acc_full0 + 8 * ab);
             }
         }
         __syncwarp();
@@ -390,12 +403,31 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         int sub_idx = 0;                            // sub-tiles stored so far by this block
         const uint32_t part_addr = smem_u32(partial);
         int local = 0;
-        if (a.splits > 1) {
+        if (split) {
             // ---- K is split over the cluster: one tile per block.  Every rank parks its partial
             // accumulator in its own shared memory; then rank r sums, in rank order, a slice of the
             // tile's token columns over all ranks and writes that slice.
             const int tile = blockIdx.x;
             const int row0 = (tile / tok_tiles) * TC_BM, tok0 = (tile % tok_tiles) * BN;
+            const int f = row0 + f_local;
+            const int out_f = GLU ? f >> 1 : f;
+            const int out_n = GLU ? a.N >> 1 : a.N;
+            const int per = (BN + a.splits - 1) / a.splits;
+            const int c_lo = (int)rank * per, c_hi = min(BN, c_lo + per);
+            // A product that begins a norm is the only one to add to its elements of the residual: what they hold is
+            // read here, while the sums are still being formed, and not by the atomic addition that would otherwise
+            // stand between a sum and its square.
+            const bool norms = MODE == OUT_F32_ACC && a.norm_gain != nullptr;
+            auto residual = [&](int cc) {
+                return norms && cc < c_hi && tok0 + cc < a.T && out_f < out_n
+                           ? __ldcg(reinterpret_cast<const float*>(a.Y) + (long)(tok0 + cc) * a.ldy + out_f) : 0.f;
+            };
+            float gain = 0.f;
+            if (norms && out_f < out_n)
+                gain = (a.norm_gain_dtype == ZLM_F32 ? reinterpret_cast<const float*>(a.norm_gain)[out_f]
+                                                     : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.norm_gain)[out_f])) +
+                       a.norm_offset;
+            float ahead = residual(c_lo + egroup);
             if (n_kb > 0) mbar_wait(acc_full0, 0, abort_flag, a.err, ERR_WAIT_ACCUM);
             asm volatile("bar.sync 2, 256;" ::: "memory");
             const bool good = *abort_flag == 0;
@@ -413,21 +445,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             }
             cluster_sync_arrive_wait();
             first_cluster_barrier_done = true;
-            const int f = row0 + f_local;
             float bias_v = 0.f;
             if (a.bias != nullptr && f < a.N)
                 bias_v = a.bias_dtype == ZLM_F32 ? reinterpret_cast<const float*>(a.bias)[f]
                                                 : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.bias)[f]);
-            const int out_f = GLU ? f >> 1 : f;
-            const int out_n = GLU ? a.N >> 1 : a.N;
-            const int per = (BN + a.splits - 1) / a.splits;
-            const int c_lo = (int)rank * per, c_hi = min(BN, c_lo + per);
             uint32_t remote[8];
 #pragma unroll
             for (int r = 0; r < 8; ++r) remote[r] = r < a.splits ? map_to_rank(part_addr, (uint32_t)r) : 0u;
-            // Up to EB tokens of this warp at a time (tiles of 64 tokens and more): their partials are all requested before the first sum,
-            // their additions to the residual all issued before the first result is used, so the latencies of
-            // the cluster's shared memory and of the returning atomics are paid once per group, not per token.
+            // Up to EB tokens of this warp at a time (tiles of 64 tokens and more): their partials are all requested before the
+            // first sum, so the latency of the cluster's shared memory is paid once per group, not per token.
             constexpr int EB = BN >= 64 ? 2 : 1;          // narrow tiles keep their registers: three blocks an SM
             if constexpr (EB == 1) {
                 for (int cc = c_lo + egroup; cc < c_hi && good; cc += 2) {
@@ -437,6 +463,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     #pragma unroll
                     for (int r = 0; r < 8; ++r)
                         part[r] = r < a.splits ? ld_cluster_f32(remote[r] + 4u * (cc * TC_BM + f_local)) : 0.f;
+                    const float before = ahead;
+                    ahead = residual(cc + 2);
                     float val = part[0];
     #pragma unroll
                     for (int r = 1; r < 8; ++r) val += part[r];
@@ -462,11 +490,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                         // sum of squares (four warps of this half of the epilogue, summed in warp order).
                         float xn = 0.f;
                         if (out_f < out_n) {
-                            xn = atomicAdd(reinterpret_cast<float*>(a.Y) + (long)tok * a.ldy + out_f, val) + val;
-                            const float g = a.norm_gain_dtype == ZLM_F32
-                                                ? reinterpret_cast<const float*>(a.norm_gain)[out_f]
-                                                : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.norm_gain)[out_f]);
-                            a.norm_hb[(long)tok * a.ld_hb + out_f] = __float2bfloat16_rn(xn * (g + a.norm_offset));
+                            xn = before + val;
+                            reinterpret_cast<float*>(a.Y)[(long)tok * a.ldy + out_f] = xn;
+                            a.norm_hb[(long)tok * a.ld_hb + out_f] = __float2bfloat16_rn(xn * gain);
                         }
                         const float sq = warp_sum(xn * xn);
                         if (lane == 0) norm_red[egroup][0][q] = sq;
@@ -483,7 +509,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                 for (int cc0 = c_lo + egroup; cc0 < c_hi && good; cc0 += 2 * EB) {
                     if (tok0 + cc0 >= a.T) break;
                     bool live[EB];
-                    float val[EB];
+                    float val[EB], before[EB];
+    #pragma unroll
+                    for (int u = 0; u < EB; ++u) before[u] = u == 0 ? ahead : residual(cc0 + 2 * u);
+                    ahead = residual(cc0 + 2 * EB);
                     float part[EB][8];
     #pragma unroll
                     for (int u = 0; u < EB; ++u) {
@@ -509,18 +538,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                         }
                         val[u] = v;
                     }
-                    float before[EB];
     #pragma unroll
                     for (int u = 0; u < EB; ++u) {
                         const int tok = tok0 + cc0 + 2 * u;
-                        before[u] = 0.f;
                         if (!live[u] || !writer || out_f >= out_n) continue;
                         if (MODE == OUT_BF16 || GLU)
                             reinterpret_cast<__nv_bfloat16*>(a.Y)[(long)tok * a.ldy + out_f] = __float2bfloat16_rn(val[u]);
                         else if (MODE == OUT_F32_ACC && a.norm_gain == nullptr)   // one adder per element: the order is fixed
                             atomicAdd(reinterpret_cast<float*>(a.Y) + (long)tok * a.ldy + out_f, val[u]);
                         else if (MODE == OUT_F32_ACC)
-                            before[u] = atomicAdd(reinterpret_cast<float*>(a.Y) + (long)tok * a.ldy + out_f, val[u]);
+                            reinterpret_cast<float*>(a.Y)[(long)tok * a.ldy + out_f] = before[u] + val[u];
                         else
                             reinterpret_cast<float*>(a.Y)[(long)tok * a.ldy + out_f] = val[u];
                     }
@@ -528,17 +555,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                         // The only adder of an element sees the finished residual value: it leaves x * gain for
                         // the product after the norm, and the tile's 128 features of a token give one partial
                         // sum of squares (four warps of this half of the epilogue, summed in warp order).
-                        float g = 0.f;
-                        if (out_f < out_n)
-                            g = (a.norm_gain_dtype == ZLM_F32
-                                     ? reinterpret_cast<const float*>(a.norm_gain)[out_f]
-                                     : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.norm_gain)[out_f])) + a.norm_offset;
     #pragma unroll
                         for (int u = 0; u < EB; ++u) {
                             float xn = 0.f;
                             if (live[u] && out_f < out_n) {
                                 xn = before[u] + val[u];
-                                a.norm_hb[(long)(tok0 + cc0 + 2 * u) * a.ld_hb + out_f] = __float2bfloat16_rn(xn * g);
+                                a.norm_hb[(long)(tok0 + cc0 + 2 * u) * a.ld_hb + out_f] = __float2bfloat16_rn(xn * gain);
                             }
                             const float sq = warp_sum(xn * xn);
                             if (lane == 0) norm_red[egroup][u][q] = sq;
@@ -554,7 +576,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                     }
                 }
             }
-        } else
+        } else if constexpr (!C::SPLIT) {
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++local) {
             const int row0 = (tile / tok_tiles) * TC_BM, tok0 = (tile % tok_tiles) * BN;
             const int ab = local & 1;
@@ -569,11 +591,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty0 + 8 * ab);
         }
-        if (a.tma_store && a.splits == 1 && warp == 2 && lane == 0) tma_store_wait_read();
+        }
+        if (a.tma_store && !split && warp == 2 && lane == 0) tma_store_wait_read();
         __syncwarp();
     }
 
-    if (a.splits > 1) {
+    if (split) {
         // every thread of every rank passes two cluster barriers: after the partials are written
         // (rank 0's epilogue passes the first one inside its loop) and after they are read
         if (!first_cluster_barrier_done) cluster_sync_arrive_wait();
@@ -906,9 +929,29 @@ static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const CUtenso
     return e == cudaSuccess ? launch_status() : (int)e;
 }
 
+// Launches that split K, tiles of at most 32 tokens: the number of stages by blocks and K blocks (see TcCfg).
+template <int BN, int MODE>
+static int launch_split(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& my, const TcArgs& a, cudaStream_t s) {
+    // two of the deep form still fit an SM: a cluster of eight finds its SMs in one part of the chip
+    constexpr int DEEP = BN == 16 ? SPLIT_K + 6 : SPLIT_K + 5;
+    if (a.grid_x * a.splits <= 148 && a.kb_per_split > 4) return launch_tc<BN, MODE, DEEP>(mw, mx, my, a, s);
+    return launch_tc<BN, MODE, SPLIT_K + 4>(mw, mx, my, a, s);
+}
+
 template <int BN>
 static int pick_mode(int mode, const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& my, const TcArgs& a,
                      cudaStream_t s) {
+    if constexpr (BN <= 32) {
+        if (a.splits > 1) {
+            switch (mode) {
+                case OUT_F32: return launch_split<BN, OUT_F32>(mw, mx, my, a, s);
+                case OUT_F32_ACC: return launch_split<BN, OUT_F32_ACC>(mw, mx, my, a, s);
+                case OUT_BF16_GLU: return launch_split<BN, OUT_BF16_GLU>(mw, mx, my, a, s);
+                case OUT_BF16_GEGLU: return launch_split<BN, OUT_BF16_GEGLU>(mw, mx, my, a, s);
+                default: return launch_split<BN, OUT_BF16>(mw, mx, my, a, s);
+            }
+        }
+    }
     switch (mode) {
         case OUT_F32: return launch_tc<BN, OUT_F32>(mw, mx, my, a, s);
         case OUT_F32_ACC: return launch_tc<BN, OUT_F32_ACC>(mw, mx, my, a, s);
@@ -1043,14 +1086,15 @@ static int gemm_tc_run(const void* X, const void* W, const void* bias, int bias_
     int s = splits;
     if (s == 0) {
         s = 1;
-        if (bn <= 64 && tiles < 148) {
-            s = (296 + tiles - 1) / tiles;                    // enough CTAs for two per SM
-            // the gated product pays for CTAs beyond one resident wave (measured at 128 tiles: 2 beats 3)
-            if (glu && s > 1 && tiles * s > 296) --s;
-            // 32 and 64 tokens: a rank's share of the reduction over the cluster grows with the tile.  Measured
-            // inside decode steps of 32 and 64 sequences (8B shapes): a product that stores does best with five
-            // ranks (48 tiles), one that adds with seven rather than eight (32 tiles).
-            if (bn >= 32 && s > (accumulate ? 7 : 5)) s = accumulate ? 7 : 5;
+        // As many blocks as are resident at once: three an SM with tiles of 16 tokens, two with wider ones; more start
+        // late and cost more than they bring (16 tokens: 16384 x 2048 gated, 128 tiles, in three parts 13.7 us, in two
+        // 16.1; 27648 x 5120 gated, 216 tiles, in two 45.1, whole 47.4; 28672 x 4096 gated, 224 tiles, whole 40.5, in
+        // two 44.2).  From 32 tokens on a rank's share of the reduction over the cluster grows with the tile, and a
+        // product that stores does best short of that (6144 x 4096, 64 tokens: five ranks 13.5 us, six 19.7).
+        if (bn <= 64) {
+            const int blocks = bn == 16 ? 3 * 148 : (glu || accumulate) ? 2 * 148 : 240;
+            s = blocks / tiles;
+            if (s < 1) s = 1;
             if (s > 8) s = 8;
             const int most = a.kb_total / 4 > 0 ? a.kb_total / 4 : 1;   // at least 4 K blocks per CTA
             if (s > most) s = most;
