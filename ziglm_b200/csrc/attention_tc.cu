@@ -734,12 +734,22 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     }
 
     // ---- consumers
+    const int half = rope.fused ? rope.rot / 2 : 0;
+    int t_angles = -1;
+    // cosines and sines of a token's position (float32 angles, as the separate kernel forms them)
+    auto angles = [&](int tok) {
+        if (t_angles >= 0) bar_consumers();
+        const float pos = (float)positions[tok];
+        for (int i = threadIdx.x; i < half; i += ATC_CONSUMERS * 32) sincosf(pos * rope.inv_freq[i], &sn_s[i], &cs_s[i]);
+        bar_consumers();
+        t_angles = tok;
+    };
+    if (half > 0) angles(t0);             // neither positions nor frequencies come from the kernel before
     pdl_wait();
     const int gid = lane >> 2, tid4 = lane & 3;
     // a slot: [group][HD] sums, then [group][2] (maximum, denominator); slots start on 16-byte boundaries
     const long slot_floats = ((long)group * (HD + 2) + 3) / 4 * 4;
-    const int half = rope.fused ? rope.rot / 2 : 0;
-    int t = t0, kvh = kvh0, it = 0, t_angles = -1;
+    int t = t0, kvh = kvh0, it = 0;
     long vi = v0_item;
     for (bool first_item = true; ; first_item = false) {
         if (!first_item && ++kvh == a.n_kv) { kvh = 0; ++t; }
@@ -753,14 +763,21 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         const int pos = positions[t];
         const int start = first_visible_key(pos, a.window);
         const int first_page = start / PAGE;
-        if (half > 0 && t != t_angles) {
-            // cosines and sines of this token's position (float32 angles, as the separate kernel forms them)
-            if (t_angles >= 0) bar_consumers();
-            for (int i = threadIdx.x; i < half; i += ATC_CONSUMERS * 32)
-                sincosf((float)pos * rope.inv_freq[i], &sn_s[i], &cs_s[i]);
-            bar_consumers();
-            t_angles = t;
+        // The new key and value, and the page they go to: asked for here, beside the queries, so that their latencies do
+        // not stand between the item's last page and its scores.  A thread takes element threadIdx.x (HD <= 128).
+        const bool brings_new = rope.fused && rope.store && j + seg == p_t && (int)threadIdx.x < HD;
+        __nv_bfloat16 new_x = __float2bfloat16_rn(0.f), new_y = new_x, new_v = new_x;
+        int new_page = 0;
+        if (brings_new) {
+            const int d = threadIdx.x;
+            const __nv_bfloat16* knew = a.q + (long)t * a.q_row_stride + (long)(a.n_heads + kvh) * HD;
+            new_page = a.block_table[(long)seq_of_token[t] * a.bt_stride + first_page + p_t - 1];
+            const int ii = d < half ? d : d < 2 * half ? d - half : d;
+            new_x = knew[ii];
+            if (d < 2 * half) new_y = knew[ii + half];
+            new_v = ((MORE && rope.values_from_keys) ? knew : knew + (long)a.n_kv * HD)[d];
         }
+        if (half > 0 && t != t_angles) angles(t);
         const __nv_bfloat16* qrow = a.q + (long)t * a.q_row_stride + (long)kvh * group * HD;
         uint32_t qf[HD / 16][4];
         load_q_frags<HD>(qf, gid < group ? qrow + gid * HD : nullptr, gid + 8 < group ? qrow + (gid + 8) * HD : nullptr,
@@ -797,10 +814,9 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                 landed = !bar_consumers_or(!landed);
                 if (landed) {
                     const int r = pos % PAGE;
-                    const __nv_bfloat16* knew = a.q + (long)t * a.q_row_stride + (long)(a.n_heads + kvh) * HD;
-                    const __nv_bfloat16* vnew = (MORE && rope.values_from_keys) ? knew : knew + (long)a.n_kv * HD;
                     float kinv = 1.0f;
                     if (MORE && rope.norm_dim > 0) {
+                        const __nv_bfloat16* knew = a.q + (long)t * a.q_row_stride + (long)(a.n_heads + kvh) * HD;
                         float ss = 0.f;
                         for (int d = lane; d < HD; d += 32) {
                             const float x = __bfloat162float(knew[d]);
@@ -808,28 +824,24 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                         }
                         kinv = 1.0f / sqrtf(warp_sum(ss) / (float)rope.norm_dim + rope.norm_eps);
                     }
-                    const long crow = ((long)a.block_table[(long)seq_of_token[t] * a.bt_stride + p] * a.n_kv + kvh) * PAGE + r;
-                    __nv_bfloat16* kdst = rope.k_pages + crow * HD;
-                    __nv_bfloat16* vdst = rope.v_pages + crow * HD;
-                    uint8_t* ktile = smem + (k0 + s * C::TILE_BYTES - base);
-                    uint8_t* vtile = smem + (v0 + s * C::TILE_BYTES - base);
-                    for (int d = threadIdx.x; d < HD; d += ATC_CONSUMERS * 32) {
+                    if (brings_new) {
+                        const int d = threadIdx.x;
+                        const long crow = ((long)new_page * a.n_kv + kvh) * PAGE + r;
                         __nv_bfloat16 kv;
                         if (d < 2 * half) {
                             const int ii = d < half ? d : d - half;
-                            const float x = __bfloat162float(knew[ii]), y = __bfloat162float(knew[ii + half]);
+                            const float x = __bfloat162float(new_x), y = __bfloat162float(new_y);
                             kv = __float2bfloat16_rn(d < half ? x * cs_s[ii] - y * sn_s[ii] : x * sn_s[ii] + y * cs_s[ii]);
                         } else if (MORE && rope.norm_dim > 0) {
-                            kv = __float2bfloat16_rn((__bfloat162float(knew[d]) * kinv) * rope.k_w[d]);
+                            kv = __float2bfloat16_rn((__bfloat162float(new_x) * kinv) * rope.k_w[d]);
                         } else {
-                            kv = knew[d];
+                            kv = new_x;
                         }
-                        const __nv_bfloat16 vv = vnew[d];
                         const uint32_t off = tile_addr(0u, r, d >> 3) + (d & 7) * 2;
-                        *reinterpret_cast<__nv_bfloat16*>(ktile + off) = kv;
-                        *reinterpret_cast<__nv_bfloat16*>(vtile + off) = vv;
-                        kdst[d] = kv;
-                        vdst[d] = vv;
+                        *reinterpret_cast<__nv_bfloat16*>(smem + (k0 + s * C::TILE_BYTES - base) + off) = kv;
+                        *reinterpret_cast<__nv_bfloat16*>(smem + (v0 + s * C::TILE_BYTES - base) + off) = new_v;
+                        rope.k_pages[crow * HD + d] = kv;
+                        rope.v_pages[crow * HD + d] = new_v;
                     }
                 }
                 bar_consumers();
