@@ -445,25 +445,54 @@ sample_kernel(float* __restrict__ logits, int V, long row_stride, SampleArgs a, 
 // The chain with 1 <= top_k <= 64 on a large vocabulary.  SP_PARTS blocks take a slice of the row each: they
 // apply the penalties of the ids in their slice, keep the scaled logits of the slice in shared memory, find
 // its maximum, its sum of exponentials and its k best candidates exactly (radix select in shared memory,
-// ties to the lower id), and leave them in scratch.  The global k best are among those: the block that
-// arrives last at the row's counter sorts the SP_PARTS * k candidates by (logit descending, id ascending),
-// forms the row's maximum and denominator from the slices' and cuts and draws as sample_kernel does.
+// ties to the lower id), sort them and leave them in scratch.  The global k best are among those: the block that
+// arrives last at the row's counter merges the SP_PARTS sorted lists pair by pair, the 64 best of every two, forms
+// the row's maximum and denominator from the slices' and cuts and draws as sample_kernel does.
+// Everything but the last sums is done by all threads: the search for the k-th value's bin (one thread walking 256
+// bins four times), the candidates' collection (runs of a thread, 16 words apart in shared memory) and the sort of all
+// 2,048 candidates were most of 222 us a call at 64 rows of 128,256.
 constexpr int SP_PARTS = 32;
 constexpr int SP_THREADS = 256;
 constexpr int SP_KMAX = 64;
-constexpr int SP_SORT = SP_PARTS * SP_KMAX;          // 2048 candidates, a power of two
+constexpr int SP_SORT = SP_PARTS * SP_KMAX;          // 2048 candidates
 
-__global__ void __launch_bounds__(SP_THREADS)
+// Larger for a larger logit (the two zeros are one), then for a lower id.
+__device__ __forceinline__ unsigned long long sp_key(float z, int id) {
+    return ((unsigned long long)orderable(__fadd_rn(z, 0.0f)) << 32) | (0xffffffffu - (unsigned)id);
+}
+__device__ __forceinline__ float sp_logit(unsigned long long key) {
+    const unsigned o = (unsigned)(key >> 32);
+    return __uint_as_float((o & 0x80000000u) ? o ^ 0x80000000u : ~o);
+}
+__device__ __forceinline__ int sp_id(unsigned long long key) { return (int)(0xffffffffu - (unsigned)key); }
+
+// The sum of v over the threads up to and including this one (256 threads); `scratch` needs 8 ints.
+__device__ __forceinline__ int sp_scan(int v, int* scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+    }
+    __syncthreads();
+    if (lane == 31) scratch[warp] = v;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) v += scratch[w];
+    return v;
+}
+
+__global__ void __launch_bounds__(SP_THREADS, 6)
 sample_parts_kernel(float* __restrict__ logits, int V, long row_stride, SampleArgs a, const int* __restrict__ history,
                     const long long* __restrict__ rng, int* __restrict__ out, int* __restrict__ counters,
                     float* __restrict__ pmax, float* __restrict__ psum, float* __restrict__ cz, int* __restrict__ cid) {
-    extern __shared__ float dyn[];
+    extern __shared__ __align__(16) float dyn[];
     __shared__ float fscratch[33];
-    __shared__ int iscratch[32];
-    __shared__ int itotal;
+    __shared__ int iscratch[8];
     __shared__ int hist[256];
+    __shared__ unsigned long long best[SP_KMAX];
+    __shared__ __align__(16) float prob[SP_KMAX];
     __shared__ unsigned prefix_s;
-    __shared__ int remaining_s;
+    __shared__ int remaining_s, ties_s;
     __shared__ int n_cand;
     __shared__ int last_s;
     const int tid = threadIdx.x, r = blockIdx.y, part = blockIdx.x;
@@ -493,6 +522,7 @@ sample_parts_kernel(float* __restrict__ logits, int V, long row_stride, SampleAr
     }
     // 1. the slice, its maximum and its sum of exponentials
     float m = -INFINITY;
+#pragma unroll 8
     for (int i = tid; i < n; i += SP_THREADS) {
         const float v = row[lo + i] * a.inv_temperature;
         z[i] = v;
@@ -502,94 +532,85 @@ sample_parts_kernel(float* __restrict__ logits, int V, long row_stride, SampleAr
     float part_sum = 0.f;
     for (int i = tid; i < n; i += SP_THREADS) part_sum += expf(z[i] - m);
     part_sum = block_sum(part_sum, fscratch);
-    // 2. the k best of the slice, exactly
+    // 2. the k best of the slice, exactly: the value of the k-th, byte by byte from the top
     const int k = min(a.top_k, n);
-    if (tid == 0) { prefix_s = 0u; remaining_s = k; }
-    __syncthreads();
+    if (tid == 0) { prefix_s = 0u; remaining_s = k; ties_s = 0; n_cand = 0; }
     for (int pass = 0; pass < 4 && k > 0; ++pass) {
         const int shift = 24 - 8 * pass;
         hist[tid] = 0;
         __syncthreads();
         const unsigned prefix = prefix_s;
+        const int remaining = remaining_s;
         const unsigned mask = pass == 0 ? 0u : (0xffffffffu << (shift + 8));
         for (int i = tid; i < n; i += SP_THREADS) {
             const unsigned key = orderable(z[i]);
             if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 0xff], 1);
         }
         __syncthreads();
-        if (tid == 0) {
-            int rem = remaining_s;
-            int b = 255;
-            for (; b > 0; --b) {
-                if (hist[b] >= rem) break;
-                rem -= hist[b];
-            }
-            prefix_s = prefix | ((unsigned)b << shift);
-            remaining_s = rem;
+        // from the top bin down: the bin in which the count reaches what remains
+        const int bin = 255 - tid, count = hist[bin];
+        const int upto = sp_scan(count, iscratch);
+        if (upto >= remaining && upto - count < remaining) {
+            prefix_s = prefix | ((unsigned)bin << shift);
+            remaining_s = remaining - (upto - count);
+            ties_s = count;
         }
         __syncthreads();
     }
+    __syncthreads();
     const unsigned kth = prefix_s;
-    const int ties_needed = remaining_s;
-    float* my_cz = cz + ((long)r * SP_PARTS + part) * SP_KMAX;
-    int* my_cid = cid + ((long)r * SP_PARTS + part) * SP_KMAX;
-    if (tid == 0) n_cand = 0;
-    __syncthreads();
-    // contiguous runs per thread, so that ties are taken in id order
-    const int run = (n + SP_THREADS - 1) / SP_THREADS;
-    const int t_lo = min(n, tid * run), t_hi = min(n, t_lo + run);
-    int my_ties = 0;
-    for (int i = t_lo; i < t_hi && k > 0; ++i) {
-        const unsigned key = orderable(z[i]);
-        if (key > kth) {
-            const int slot = atomicAdd(&n_cand, 1);
-            my_cz[slot] = z[i];
-            my_cid[slot] = lo + i;
-        } else if (key == kth) {
-            ++my_ties;
+    const int ties_needed = remaining_s;                   // of the values equal to the k-th, the first ones by id
+    const bool all_ties = ties_s == ties_needed;
+    if (k > 0) {
+        for (int i = tid; i < n; i += SP_THREADS) {
+            const unsigned key = orderable(z[i]);
+            if (key > kth || (all_ties && key == kth)) best[atomicAdd(&n_cand, 1)] = sp_key(z[i], lo + i);
         }
-    }
-    // exclusive scan of the ties over the 256 threads (8 warps)
-    int tie_rank;
-    {
-        const int lane = tid & 31, warp = tid >> 5;
-        int inc = my_ties;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += v;
-        }
-        __syncthreads();
-        if (lane == 31) iscratch[warp] = inc;
-        __syncthreads();
-        int before = 0;
-        for (int w = 0; w < warp; ++w) before += iscratch[w];
-        tie_rank = before + inc - my_ties;
-    }
-    __syncthreads();
-    const int n_above = n_cand;
-    {
-        int rank = tie_rank;
-        for (int i = t_lo; i < t_hi && rank < ties_needed; ++i) {
-            if (orderable(z[i]) == kth) {
-                my_cz[n_above + rank] = z[i];
-                my_cid[n_above + rank] = lo + i;
-                ++rank;
+        if (!all_ties) {
+            // contiguous runs per thread, so that ties are taken in id order
+            const int run = (n + SP_THREADS - 1) / SP_THREADS;
+            const int t_lo = min(n, tid * run), t_hi = min(n, t_lo + run);
+            int my_ties = 0;
+            for (int i = t_lo; i < t_hi; ++i) my_ties += orderable(z[i]) == kth;
+            int rank = sp_scan(my_ties, iscratch) - my_ties;           // its barriers also complete n_cand
+            const int n_above = n_cand;
+            for (int i = t_lo; i < t_hi && rank < ties_needed; ++i) {
+                if (orderable(z[i]) == kth) {
+                    best[n_above + rank] = sp_key(z[i], lo + i);
+                    ++rank;
+                }
             }
         }
     }
-    for (int i = k + tid; i < SP_KMAX; i += SP_THREADS) { my_cz[i] = -INFINITY; my_cid[i] = 0x7fffffff; }
-    if (tid == 0) { pmax[r * SP_PARTS + part] = m; psum[r * SP_PARTS + part] = part_sum; }
-    __threadfence();
+    for (int i = k + tid; i < SP_KMAX; i += SP_THREADS) best[i] = sp_key(-INFINITY, 0x7fffffff);
     __syncthreads();
-    if (tid == 0) last_s = atomicAdd(&counters[r], 1) == SP_PARTS - 1;
+    // 3. one warp sorts them, largest first, and leaves them in scratch
+    if (tid < 32) {
+        for (int size = 2; size <= SP_KMAX; size <<= 1) {
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                const int i = 2 * tid - (tid & (stride - 1)), j = i + stride;
+                const unsigned long long x = best[i], y = best[j];
+                if ((x < y) == ((i & size) == 0)) { best[i] = y; best[j] = x; }
+                __syncwarp();
+            }
+        }
+        for (int i = tid; i < SP_KMAX; i += 32) {
+            cz[((long)r * SP_PARTS + part) * SP_KMAX + i] = sp_logit(best[i]);
+            cid[((long)r * SP_PARTS + part) * SP_KMAX + i] = sp_id(best[i]);
+        }
+        if (tid == 0) { pmax[r * SP_PARTS + part] = m; psum[r * SP_PARTS + part] = part_sum; }
+        __threadfence();
+    }
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        last_s = atomicAdd(&counters[r], 1) == SP_PARTS - 1;
+    }
     __syncthreads();
     if (!last_s) return;
     __threadfence();
 
     // ---- the last block of the row: maximum and denominator of the row, in slice order
-    float* sz = dyn;                                       // [SP_SORT]
-    int* sid = reinterpret_cast<int*>(dyn + SP_SORT);      // [SP_SORT]
     float row_max, denom;
     {
         float mp = tid < SP_PARTS ? __ldcg(&pmax[r * SP_PARTS + tid]) : -INFINITY;
@@ -597,53 +618,65 @@ sample_parts_kernel(float* __restrict__ logits, int V, long row_stride, SampleAr
         float sp = tid < SP_PARTS ? __ldcg(&psum[r * SP_PARTS + tid]) * expf(mp - row_max) : 0.f;
         denom = block_sum(sp, fscratch);
     }
-    for (int i = tid; i < SP_SORT; i += SP_THREADS) {
-        sz[i] = __ldcg(&cz[(long)r * SP_SORT + i]);
-        sid[i] = __ldcg(&cid[(long)r * SP_SORT + i]);
-    }
+    unsigned long long* keys = reinterpret_cast<unsigned long long*>(dyn);         // [SP_PARTS][SP_KMAX]
+#pragma unroll
+    for (int i = 0; i < SP_SORT; i += SP_THREADS)
+        keys[i + tid] = sp_key(__ldcg(&cz[(long)r * SP_SORT + i + tid]), __ldcg(&cid[(long)r * SP_SORT + i + tid]));
     __syncthreads();
-    for (int size = 2; size <= SP_SORT; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = tid; i < SP_SORT; i += SP_THREADS) {
-                const int j = i ^ stride;
-                if (j > i) {
-                    const bool up = (i & size) == 0;
-                    const float zi = sz[i], zj = sz[j];
-                    const int ii = sid[i], ij = sid[j];
-                    const bool i_first = zi > zj || (zi == zj && ii < ij);
-                    if (i_first != up) { sz[i] = zj; sz[j] = zi; sid[i] = ij; sid[j] = ii; }
-                }
+    for (int lists = SP_PARTS / 2; lists > 0; lists >>= 1) {
+        // list p keeps the 64 best of itself and of list p + lists: the larger of a[i] and b[63 - i] are those, first
+        // rising and then falling or the other way round, which six rounds put in order
+        for (int x = tid; x < lists * SP_KMAX; x += SP_THREADS) {
+            const unsigned long long other = keys[(x / SP_KMAX + lists) * SP_KMAX + SP_KMAX - 1 - x % SP_KMAX];
+            if (other > keys[x]) keys[x] = other;
+        }
+        __syncthreads();
+        for (int stride = SP_KMAX / 2; stride > 0; stride >>= 1) {
+            for (int x = tid; x < lists * (SP_KMAX / 2); x += SP_THREADS) {
+                const int i = 2 * x - (x & (stride - 1)), j = i + stride;
+                const unsigned long long u = keys[i], w = keys[j];
+                if (u < w) { keys[i] = w; keys[j] = u; }
             }
             __syncthreads();
         }
     }
+    if (tid < SP_KMAX) prob[tid] = expf(sp_logit(keys[tid]) - row_max) / denom;
+    __syncthreads();
     if (tid == 0) {
+        const float* p = prob;                             // no loop breaks off: the reads run ahead of the sums
         const float u = uniform01((unsigned long long)rng[2 * r], (unsigned long long)rng[2 * r + 1]);
         int nn = min(a.top_k, V);
-        const float p0 = expf(sz[0] - row_max) / denom;
         if (a.min_p > 0.f) {
-            const float thresh = p0 * a.min_p;
-            for (int i = 0; i < nn; ++i) {
-                if (expf(sz[i] - row_max) / denom < thresh) { nn = max(1, i); break; }
-            }
+            const float thresh = p[0] * a.min_p;
+            int cut = nn;
+#pragma unroll 16
+            for (int i = SP_KMAX - 1; i >= 0; --i)
+                if (i < nn && p[i] < thresh) cut = max(1, i);
+            nn = cut;
         }
         if (a.top_p < 1.0f) {
             float cum = 0.f;
-            for (int i = 0; i < nn; ++i) {
-                cum += expf(sz[i] - row_max) / denom;
-                if (cum >= a.top_p) { nn = i + 1; break; }
+            int cut = nn;
+#pragma unroll 16
+            for (int i = 0; i < SP_KMAX; ++i) {
+                cum += p[i];
+                if (i < cut && cum >= a.top_p) cut = i + 1;
             }
+            nn = cut;
         }
         float total = 0.f;
-        for (int i = 0; i < nn; ++i) total += expf(sz[i] - row_max) / denom;
+#pragma unroll 16
+        for (int i = 0; i < SP_KMAX; ++i)
+            if (i < nn) total += p[i];
         const float rr = u * total;
         float running = 0.f;
-        int pick = sid[0];
-        for (int i = 0; i < nn; ++i) {
-            running += expf(sz[i] - row_max) / denom;
-            if (rr <= running) { pick = sid[i]; break; }
+        int pick = -1;
+#pragma unroll 16
+        for (int i = 0; i < SP_KMAX; ++i) {
+            running += p[i];
+            if (pick < 0 && i < nn && rr <= running) pick = i;
         }
-        out[r] = pick;
+        out[r] = sp_id(keys[pick < 0 ? 0 : pick]);
         counters[r] = 0;
     }
 }
