@@ -55,6 +55,37 @@ def test_gemm_tc_split_k_is_exact_in_order(K, splits, T):
     assert torch.allclose(out.cpu(), base + ref_product(x, w), atol=2e-3, rtol=1e-3)
 
 
+# Split launches by stage count: four stages (4 K blocks a part and fewer), five or six (one block an SM, 5 and more K
+# blocks a part), a last part that is shorter, more tiles than are split; and the first sizes of the wider tiles.
+@pytest.mark.parametrize("T", [1, 16, 17, 32, 64, 65, 128])
+@pytest.mark.parametrize("N,K_", [(256, 2048), (384, 2560), (2048, 8192), (1000, 1096), (28416, 512), (28544, 512)])
+def test_gemm_tc_split_stages(K, T, N, K_):
+    x, w, b = rnd((T, K_), BF, seed=51).to(DEV), rnd((N, K_), BF, 0.05, seed=52).to(DEV), rnd((N,), BF, seed=53).to(DEV)
+    base = rnd((T, N), torch.float32, seed=54).to(DEV)
+    want = x.double() @ w.double().t()
+    # a product of two bf16 is exact in float32; every addition loses at most one unit of the last place (rounded or cut)
+    bound = (K_ + 2) * 2.0 ** -23 * (x.abs().double() @ w.abs().double().t() + base.abs().double() + b.abs().double())
+    out = torch.full((T, N), 7.0, device=DEV)
+    assert K.gemm_tc(x, w, out, bias=b)
+    assert ((out.double() - (want + b.double())).abs() <= bound).all()
+    acc = base.clone()
+    assert K.gemm_tc(x, w, acc, accumulate=True)
+    assert ((acc.double() - (want + base.double())).abs() <= bound).all()
+    if T <= 64:
+        # the norm rides on the sum: x * gain and the sums of squares come from the residual the launch leaves
+        gain, hb = rnd((N,), torch.float32, seed=55).to(DEV), torch.empty(T, N, dtype=BF, device=DEV)
+        ssq, res = torch.zeros(T, -(-N // 128), device=DEV), base.clone()
+        if K.gemm_tc(x, w, res, accumulate=True, norm_out=(gain, 0.0, hb, ssq)) == 2:
+            assert torch.equal(hb, (res * gain).to(BF))
+            assert torch.allclose(ssq.sum(1), (res * res).sum(1), rtol=N * 2.0 ** -23)
+        assert ((res.double() - (want + base.double())).abs() <= bound).all()
+    gated = torch.full((T, N // 2), 7.0, dtype=BF, device=DEV)
+    assert K.gemm_tc(x, w, gated, glu="silu")
+    g, u = want[:, 0::2], want[:, 1::2]
+    assert torch.allclose(gated.double(), torch.nn.functional.silu(g) * u, atol=3e-2, rtol=2e-2)
+    assert K.gemm_tc_status() == 0
+
+
 # Steps of more than 128 tokens: the kernel that pairs two CTAs on tiles of 256 weight rows (splits=0) and the
 # one-CTA kernel (splits=1), in every output mode.  Shapes: one pair tile; an odd number of row tiles (the last
 # pair is half empty); a ragged K and N; many tiles per pair and a long K; few tiles and a long K (the
