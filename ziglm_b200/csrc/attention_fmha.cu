@@ -385,7 +385,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         constexpr uint32_t idesc_o = idesc_bf16_b_mn(FM_BQ, HD);          // O: 128 x head_dim, K = 16 keys
         const uint64_t dq = smem_desc_sw128(q_smem), dk = smem_desc_sw128(k_smem);
         const uint64_t dv = smem_desc_sw128_mn(v_smem, FM_PAGE * 128);
-        bool alive = mbar_wait(q_full, 0, abort_flag, a.err, ERR_FM_Q);
+        bool alive = warp_wait(q_full, 0, abort_flag, a.err, ERR_FM_Q);
         // step j: for each tile first P V of step j - 1, then the scores of step j
         for (int j = 0; j <= n_steps && alive; ++j) {
 #pragma unroll
@@ -396,12 +396,11 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     const int np = pages_of(jj);
                     const uint32_t tmem_o = tmem_base + C::O_COL + t * HD;
                     const uint32_t tmem_p = tmem_base + C::S_COL + t * FM_KEYS;
-                    alive = mbar_wait(v_full0 + 8 * sv, (jj / C::NV) & 1, abort_flag, a.err, ERR_FM_KV);
+                    alive = warp_wait(v_full0 + 8 * sv, (jj / C::NV) & 1, abort_flag, a.err, ERR_FM_KV);
 #pragma unroll
                     for (int pg = 0; pg < FM_NP; ++pg) {
                         if (pg < np) {
-                            alive = alive && mbar_wait(p_full0 + 8 * (t * FM_NP + pg), lt & 1, abort_flag, a.err, ERR_FM_P);
-                            alive = __all_sync(0xffffffffu, alive);
+                            alive = alive && warp_wait(p_full0 + 8 * (t * FM_NP + pg), lt & 1, abort_flag, a.err, ERR_FM_P);
                             tc_fence_after_sync();
                             if (alive && elect_one()) {
 #pragma unroll
@@ -416,8 +415,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 }
                 if (alive && j < n_steps && runs(t, j)) {
                     const int sk = j % C::NK;
-                    alive = mbar_wait(k_full0 + 8 * sk, (j / C::NK) & 1, abort_flag, a.err, ERR_FM_KV);
-                    alive = __all_sync(0xffffffffu, alive);
+                    alive = warp_wait(k_full0 + 8 * sk, (j / C::NK) & 1, abort_flag, a.err, ERR_FM_KV);
                     tc_fence_after_sync();
                     const uint32_t tmem_s = tmem_base + C::S_COL + t * FM_KEYS;
                     const uint32_t idesc_s = pages_of(j) >= FM_NP ? idesc_s2 : idesc_s1;

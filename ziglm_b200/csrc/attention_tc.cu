@@ -324,7 +324,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         for (int lp = page_lo; lp < page_hi; ++lp, ++it) {
             const int p = lp < kept_pages ? lp : lp + skip_by;
             const int s = it % C::STAGES;
-            if (!mbar_wait(full0 + 8 * s, (it / C::STAGES) & 1, abort_flag, a.err, ERR_ATT_FULL)) break;
+            if (!warp_wait(full0 + 8 * s, (it / C::STAGES) & 1, abort_flag, a.err, ERR_ATT_FULL)) break;
             if (p * PAGE >= start && p * PAGE + PAGE - 1 <= pos) {
                 page_step<HD, 2, true, SLOPES>(qf, k0 + s * C::TILE_BYTES, v0 + s * C::TILE_BYTES, warp * 16, p * PAGE + warp * 16,
                                        pos, pos, start, start, a.scale_log2, a.cap_in2, a.cap_log2, m, l, o, lane, slope2);
@@ -806,7 +806,7 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
             for (int i = 0; i < 4; ++i) o[n][i] = 0.f;
         for (int i = 0; i < seg; ++i, ++it) {
             const int s = it % C::STAGES;
-            bool landed = mbar_wait(full0 + 8 * s, (it / C::STAGES) & 1, abort_flag, a.err, ERR_ATT_FULL);
+            bool landed = warp_wait(full0 + 8 * s, (it / C::STAGES) & 1, abort_flag, a.err, ERR_ATT_FULL);
             const int p = first_page + j + i;
             if (rope.fused && rope.store && j + i == p_t - 1) {
                 // The page of position pos: its row pos % 64 is not in the cache yet.  The new key (rotated)
@@ -1105,7 +1105,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
     int it = 0;
     for (int p = page_lo; p < page_hi; ++p, ++it) {
         const int s = it % C::STAGES;
-        if (!mbar_wait(full0 + 8 * s, (it / C::STAGES) & 1, abort_flag, a.err, ERR_ATT_FULL)) break;
+        if (!warp_wait(full0 + 8 * s, (it / C::STAGES) & 1, abort_flag, a.err, ERR_ATT_FULL)) break;
         const bool needed = w_first <= pos_last && p * PAGE <= w_last && p * PAGE + PAGE - 1 >= w_start;
         if (needed) {
             // a page every row of the warp sees whole needs no masks (rows beyond the sequence never store)

@@ -357,12 +357,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             for (int tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x, ++local) {
                 const int ab = local & 1;
                 // the epilogue must have emptied this accumulator (two tiles ago)
-                alive = __all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * ab, ((local >> 1) & 1) ^ 1u, abort_flag, a.err, ERR_WAIT_ACCUM));
+                alive = warp_wait(acc_empty0 + 8 * ab, ((local >> 1) & 1) ^ 1u, abort_flag, a.err, ERR_WAIT_ACCUM);
                 if (!alive) break;
                 tc_fence_after_sync();
                 const uint32_t tmem_d = tmem_base + ab * C::ACC_COLS;
                 for (int kb = 0; kb < n_kb; ++kb) {
-                    alive = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, parity, abort_flag, a.err, ERR_WAIT_FULL));
+                    alive = warp_wait(full0 + 8 * s, parity, abort_flag, a.err, ERR_WAIT_FULL);
                     if (!alive) break;
                     tc_fence_after_sync();
                     if (elect_one()) {
@@ -759,12 +759,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 const int n_kb = min(kb_per, a.kb_total - (unit / n_tiles) * kb_per);
                 const int ab = local & 1;
                 // the epilogues of both CTAs must have emptied this accumulator (two units ago)
-                alive = __all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * ab, ((local >> 1) & 1) ^ 1u, abort_flag, a.err, ERR_WAIT_ACCUM));
+                alive = warp_wait(acc_empty0 + 8 * ab, ((local >> 1) & 1) ^ 1u, abort_flag, a.err, ERR_WAIT_ACCUM);
                 if (!alive) break;
                 tc_fence_after_sync();
                 const uint32_t tmem_d = tmem_base + ab * C::ACC_COLS;
                 for (int kb = 0; kb < n_kb; ++kb) {
-                    alive = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, parity, abort_flag, a.err, ERR_WAIT_FULL));
+                    alive = warp_wait(full0 + 8 * s, parity, abort_flag, a.err, ERR_WAIT_FULL);
                     if (!alive) break;
                     tc_fence_after_sync();
                     if (elect_one()) {

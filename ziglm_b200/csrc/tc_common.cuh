@@ -70,6 +70,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return false;
 }
 
+// The same wait by a whole warp: every lane gets the same answer, also when the polls run out in some lanes only, so that
+// the warp may branch on it and still meet in votes, shuffles and barriers.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, err, code));
+}
+
 // True in one lane of the warp, the same one each time; the whole warp calls it.
 __device__ __forceinline__ bool elect_one() {
     uint32_t e;
