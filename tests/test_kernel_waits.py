@@ -53,3 +53,18 @@ def test_a_warp_that_branches_on_a_wait_branches_as_one(name):
         assert unused, f"{name}:{line}: the lanes of a warp may take different ways: {statement.strip()}"
     for line, statement, headers in uses(text, r"produce_pages<"):
         assert one_lane(statement, headers), f"{name}:{line}"
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_warps_that_meet_at_barriers_read_the_abort_flag_as_one(name):
+    """The flag may be set between two warps' reads of it: what several warps do next is decided by a barrier that ORs what
+    they read.  A read stands where one lane runs alone, in such a barrier, or where the warp only returns."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = f.read()
+    for line, statement, headers in uses(text, r"\*abort_flag\b(?!\s*=[^=])"):
+        if one_lane(statement, headers) or any("mbar_wait(" in h or "produce_pages(" in h for h in headers):
+            continue
+        if re.search(r"\bbar_(consumers_)?or(<[^>]*>)?\($", statement):
+            continue
+        after = text.splitlines()[line - 1].split("*abort_flag", 1)[1]
+        assert re.match(r"\) return;", after), f"{name}:{line}: warps may decide differently: {statement.strip()}"

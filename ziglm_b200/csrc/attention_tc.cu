@@ -505,13 +505,7 @@ static inline FlatSizes flat_sizes(int group, int T) {
 __device__ __forceinline__ void bar_consumers() { asm volatile("bar.sync 1, %0;" ::"n"(ATC_CONSUMERS * 32) : "memory"); }
 
 // Barrier of the consumer warps that also tells every one of them whether any passed true.
-__device__ __forceinline__ bool bar_consumers_or(bool v) {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(r) : "r"((uint32_t)v), "n"(ATC_CONSUMERS * 32) : "memory");
-    return r != 0;
-}
+__device__ __forceinline__ bool bar_consumers_or(bool v) { return bar_or<1, ATC_CONSUMERS * 32>(v); }
 
 // What the flat kernel does for the step's new token itself when the rotation and the cache write are
 // not left to a kernel before it.  The rows of q are then [q heads | k heads | v heads] as the fused
@@ -846,7 +840,11 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                 }
                 bar_consumers();
             }
-            if (!landed) break;
+            if (!landed) {
+                if (i >= seg - 1) break;
+                i = seg - 2;               // a wait ran out: on to the item's last page, whose barriers the other warps may come to
+                continue;
+            }
             if (p * PAGE >= start && p * PAGE + PAGE - 1 <= pos)
                 page_step<HD, 2, true, MORE>(qf, k0 + s * C::TILE_BYTES, v0 + s * C::TILE_BYTES, warp * 16, p * PAGE + warp * 16,
                                        pos, pos, start, start, a.scale_log2, a.cap_in2, a.cap_log2, m, l, o, lane, slope2);

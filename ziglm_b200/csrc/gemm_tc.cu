@@ -429,8 +429,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
                        a.norm_offset;
             float ahead = residual(c_lo + egroup);
             if (n_kb > 0) mbar_wait(acc_full0, 0, abort_flag, a.err, ERR_WAIT_ACCUM);
-            asm volatile("bar.sync 2, 256;" ::: "memory");
-            const bool good = *abort_flag == 0;
+            const bool good = !bar_or<2, 256>(*abort_flag != 0);
             tc_fence_after_sync();
             const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
             if (good) {
@@ -581,8 +580,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             const int row0 = (tile / tok_tiles) * TC_BM, tok0 = (tile % tok_tiles) * BN;
             const int ab = local & 1;
             if (n_kb > 0) mbar_wait(acc_full0 + 8 * ab, (local >> 1) & 1, abort_flag, a.err, ERR_WAIT_ACCUM);
-            asm volatile("bar.sync 2, 256;" ::: "memory");     // the four warps go on together or not at all
-            if (*abort_flag) break;
+            if (bar_or<2, 256>(*abort_flag != 0)) break;       // the eight warps go on together or not at all
             tc_fence_after_sync();
             store_tile<C, BN, MODE>(a, &tmap_y, tmem_base + ab * C::ACC_COLS, row0, tok0, inv_s, stage_base, stage_out,
                                     sub_idx);
@@ -790,8 +788,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             const int row0 = (tile / tok_tiles) * 2 * TC_BM + (int)rank * TC_BM, tok0 = (tile % tok_tiles) * BN;
             const int ab = local & 1;
             mbar_wait(acc_full0 + 8 * ab, (local >> 1) & 1, abort_flag, a.err, ERR_WAIT_ACCUM);
-            asm volatile("bar.sync 2, 256;" ::: "memory");     // the eight warps go on together or not at all
-            if (*abort_flag) break;
+            if (bar_or<2, 256>(*abort_flag != 0)) break;       // the eight warps go on together or not at all
             tc_fence_after_sync();
             if (row0 < a.N)                                    // an odd number of row tiles leaves the last pair half empty
                 store_tile<C, BN, MODE>(a, &tmap_y, tmem_base + ab * C::ACC_COLS, row0, tok0, nullptr, stage_base,

@@ -83,6 +83,16 @@ __device__ __forceinline__ bool elect_one() {
     return e != 0;
 }
 
+// Barrier ID of N threads that also tells every one of them whether any passed true: warps that meet at barriers later on
+// decide here, together, whether they go on (each reading the abort flag by itself could see it at different times).
+template <int ID, int N> __device__ __forceinline__ bool bar_or(bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, %2, %3, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(r) : "r"((uint32_t)v), "n"(ID), "n"(N) : "memory");
+    return r != 0;
+}
+
 // 2-D TMA tile load into shared memory; completion is signalled on `bar` in bytes.
 // x is the innermost (contiguous) coordinate and must be a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
