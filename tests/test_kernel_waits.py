@@ -68,3 +68,15 @@ def test_warps_that_meet_at_barriers_read_the_abort_flag_as_one(name):
             continue
         after = text.splitlines()[line - 1].split("*abort_flag", 1)[1]
         assert re.match(r"\) return;", after), f"{name}:{line}: warps may decide differently: {statement.strip()}"
+
+
+def test_prompt_attention_asks_for_no_more_registers_than_a_build_has():
+    """The prompt attention's warps share out again what a block was launched with; asking for more than that waits for good.
+    A build of fewer registers a thread than the split needs is refused before the launch (the caller has another kernel)."""
+    from ziglm_b200 import csrc
+    fit = csrc.load("attention_fmha").zlm_attention_fmha_shares_fit
+    assert fit(168) == 1
+    assert fit(160) == 0 and fit(128) == 0
+    with open(os.path.join(CSRC, "attention_fmha.cu")) as f:
+        launch = f.read().split("static int fm_launch(", 1)[1]
+    assert launch.index("fm_shares_fit(built.numRegs)") < launch.index("launch_pdl(")

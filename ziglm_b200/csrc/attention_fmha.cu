@@ -45,9 +45,11 @@ constexpr int FM_NP = 2;             // pages per step
 constexpr int FM_KEYS = FM_PAGE * FM_NP;
 constexpr int FM_THREADS = 384;      // a warpgroup with the TMA warp and the MMA warp, then one of softmax warps per tile
 // Registers a thread after the split: what the block was launched with (168 x 384) is shared out again, so that a
-// softmax thread keeps its row of 128 scores in registers (with 168 it spilled some of them every step).
+// softmax thread keeps most of its row of 128 scores in registers.
 constexpr int FM_REGS_ISSUE = 88, FM_REGS_SOFTMAX = 208;
-static_assert(FM_REGS_ISSUE + 2 * FM_REGS_SOFTMAX <= 3 * 168, "the shares must fit what the block was launched with");
+// Whether a kernel of that many registers a thread may run: asking for more than the block was launched with waits for
+// good, so the launch asks the compiled kernel first.
+static bool fm_shares_fit(int regs_at_launch) { return FM_REGS_ISSUE + 2 * FM_REGS_SOFTMAX <= 3 * regs_at_launch; }
 constexpr int ERR_FM_ALIGN = 20, ERR_FM_Q = 21, ERR_FM_KV = 22, ERR_FM_S = 23, ERR_FM_P = 24, ERR_FM_O = 25, ERR_FM_EMPTY = 26;
 
 template <int HD> struct FmCfg {
@@ -591,7 +593,11 @@ static int fm_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
                      cudaStream_t stream) {
     static bool done = false;
     if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(fmha_prefill_kernel<HD, SLOPES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncAttributes built;
+        cudaError_t e = cudaFuncGetAttributes(&built, fmha_prefill_kernel<HD, SLOPES>);
+        if (e != cudaSuccess) return (int)e;
+        if (!fm_shares_fit(built.numRegs)) return ZLM_ERR_UNSUPPORTED;
+        e = cudaFuncSetAttribute(fmha_prefill_kernel<HD, SLOPES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              FmCfg<HD>::SMEM);
         if (e != cudaSuccess) return (int)e;
         e = cudaFuncSetAttribute(fmha_prefill_kernel<HD, SLOPES>, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -654,6 +660,9 @@ ZLM_EXPORT int zlm_attention_prefill_fmha(const void* q, long q_row_stride, long
         return hd == 128 ? fm_launch<128, true>(mq, mk, mv, a, grid, stream) : fm_launch<64, true>(mq, mk, mv, a, grid, stream);
     return hd == 128 ? fm_launch<128, false>(mq, mk, mv, a, grid, stream) : fm_launch<64, false>(mq, mk, mv, a, grid, stream);
 }
+
+// Whether the kernel's split of registers fits a build of that many registers a thread (host only).
+ZLM_EXPORT int zlm_attention_fmha_shares_fit(int regs_at_launch) { return fm_shares_fit(regs_at_launch) ? 1 : 0; }
 
 ZLM_EXPORT int zlm_attention_fmha_status(int* out) {
     int* w = fm_error_word();

@@ -177,6 +177,7 @@ _PROTOTYPES = {
                                        c_float, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                        c_void_p, c_long, c_int, c_void_p],
         "zlm_attention_fmha_status": [c_void_p],
+        "zlm_attention_fmha_shares_fit": [c_int],
         "zlm_attention_fmha_wait_selftest": [c_int, c_void_p, c_void_p],
     },
     "gemm_tc": {
