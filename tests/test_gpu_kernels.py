@@ -505,6 +505,40 @@ def test_sample_distribution_and_ties(K):
     assert set(out.tolist()) == {0, 1, 2}
 
 
+def coarse_logits(kind, V):
+    """A row of few distinct logits: ties wherever the sampler may cut."""
+    g = torch.Generator().manual_seed(31)
+    per = -(-V // 32)                                                  # ids of a slice of the sliced kernel
+    if kind == "equal":
+        return torch.zeros(V)
+    if kind == "border":                                               # more equal logits than a top_k, over several slices
+        z = torch.full((V,), -2.0)
+        z[2 * per - 2:2 * per + 90] = 1.5
+        return z
+    if kind == "few":                                                  # fewer candidates than a top_k
+        z = torch.full((V,), -math.inf)
+        z[torch.tensor([3, V // 2, V // 2 + 1, V - 2, V - 1])] = torch.tensor([1.0, 0.5, 1.0, 0.0, 0.5])
+        return z
+    z = torch.randint(-3, 4, (V,), generator=g).float() * 0.5
+    if kind == "holes":
+        z[per:3 * per] = -math.inf                                     # two slices of nothing
+    return z
+
+
+@pytest.mark.parametrize("kind", ["equal", "coarse", "border", "few", "holes"])
+@pytest.mark.parametrize("V,top_k", [(v, k) for v in (128, 1001, 4099) for k in (1, 40, 64, 100)] + [(128, 0), (1001, 0)])
+def test_sample_among_ties_draws_as_the_plain_chain(K, kind, V, top_k):
+    """Ties go to the lower id wherever they lie (inside a slice of the row, across slices, at the k-th value) and -inf weighs
+    nothing, also where a whole slice or all but a few ids hold it.  top_k <= 64 runs the sliced kernel, 100 and 0 the block
+    a row.  (The cut at 0.87 lies between two sums of these probabilities.)"""
+    from ziglm_b200.sampling import uniform01
+    row, n = coarse_logits(kind, V), 8
+    rng = torch.tensor([[5, c] for c in range(n)], dtype=torch.int64)
+    out = torch.empty(n, dtype=torch.int32, device=DEV)
+    K.sample(row.repeat(n, 1).to(DEV), out, rng.to(DEV), 1.0, top_k, 0.87, 0.0)
+    assert out.tolist() == [P.sample(row, uniform01(5, c), 1.0, top_k, 0.87, 0.0) for c in range(n)]
+
+
 def test_sample_penalties(K):
     logits = torch.tensor([[2.0, -2.0, 1.0, 0.0]])
     hist = torch.tensor([[-1, 0, 1, 0]], dtype=torch.int32)

@@ -529,8 +529,9 @@ sample_parts_kernel(float* __restrict__ logits, int V, long row_stride, SampleAr
         m = fmaxf(m, v);
     }
     m = block_max(m, fscratch);
+    const float from = m == -INFINITY ? 0.f : m;          // a slice of nothing but -inf: its exponentials are zeros, not -inf + inf
     float part_sum = 0.f;
-    for (int i = tid; i < n; i += SP_THREADS) part_sum += expf(z[i] - m);
+    for (int i = tid; i < n; i += SP_THREADS) part_sum += expf(z[i] - from);
     part_sum = block_sum(part_sum, fscratch);
     // 2. the k best of the slice, exactly: the value of the k-th, byte by byte from the top
     const int k = min(a.top_k, n);
