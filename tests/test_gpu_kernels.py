@@ -515,6 +515,11 @@ def coarse_logits(kind, V):
         z = torch.full((V,), -2.0)
         z[2 * per - 2:2 * per + 90] = 1.5
         return z
+    if kind == "zeros":                                                # more than a top_k of either sign, one tie
+        z = torch.full((V,), -1.0)
+        z[::2] = 0.0
+        z[torch.rand(V, generator=g) < 0.25] = -0.0
+        return z
     if kind == "few":                                                  # fewer candidates than a top_k
         z = torch.full((V,), -math.inf)
         z[torch.tensor([3, V // 2, V // 2 + 1, V - 2, V - 1])] = torch.tensor([1.0, 0.5, 1.0, 0.0, 0.5])
@@ -525,12 +530,12 @@ def coarse_logits(kind, V):
     return z
 
 
-@pytest.mark.parametrize("kind", ["equal", "coarse", "border", "few", "holes"])
+@pytest.mark.parametrize("kind", ["equal", "coarse", "border", "zeros", "few", "holes"])
 @pytest.mark.parametrize("V,top_k", [(v, k) for v in (128, 1001, 4099) for k in (1, 40, 64, 100)] + [(128, 0), (1001, 0)])
 def test_sample_among_ties_draws_as_the_plain_chain(K, kind, V, top_k):
-    """Ties go to the lower id wherever they lie (inside a slice of the row, across slices, at the k-th value) and -inf weighs
-    nothing, also where a whole slice or all but a few ids hold it.  top_k <= 64 runs the sliced kernel, 100 and 0 the block
-    a row.  (The cut at 0.87 lies between two sums of these probabilities.)"""
+    """Ties go to the lower id wherever they lie (inside a slice of the row, across slices, at the k-th value), +0 and -0 tie,
+    and -inf weighs nothing, also where a whole slice or all but a few ids hold it.  top_k <= 64 runs the sliced kernel, 100
+    and 0 the block a row.  (The cut at 0.87 lies between two sums of these probabilities.)"""
     from ziglm_b200.sampling import uniform01
     row, n = coarse_logits(kind, V), 8
     rng = torch.tensor([[5, c] for c in range(n)], dtype=torch.int64)

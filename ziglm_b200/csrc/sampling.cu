@@ -41,6 +41,11 @@ __device__ __forceinline__ float uniform01(unsigned long long seed, unsigned lon
     return (float)(h >> 40) * (1.0f / 16777216.0f);   // 24 bits, [0, 1)
 }
 
+// A scaled logit.  The sum makes one zero of the two: they have the same probability, and the order below would put +0 first.
+__device__ __forceinline__ float scaled(float logit, float inv_temperature) {
+    return __fadd_rn(__fmul_rn(logit, inv_temperature), 0.0f);
+}
+
 // order-preserving map from float to unsigned
 __device__ __forceinline__ unsigned orderable(float f) {
     const unsigned u = __float_as_uint(f);
@@ -215,13 +220,13 @@ sample_kernel(float* __restrict__ logits, int V, long row_stride, SampleArgs a, 
 
     // 1. scaled logits, their max, the softmax denominator
     float m = -INFINITY;
-    for (int i = tid; i < V; i += SAMPLE_THREADS) m = fmaxf(m, row[i] * a.inv_temperature);
+    for (int i = tid; i < V; i += SAMPLE_THREADS) m = fmaxf(m, scaled(row[i], a.inv_temperature));
     m = block_max(m, fscratch);
     // contiguous chunks from here on, so that running sums follow the id order
     const int chunk = (V + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
     const int lo = min(V, tid * chunk), hi = min(V, lo + chunk);
     float part = 0.f;
-    for (int i = lo; i < hi; ++i) part += expf(row[i] * a.inv_temperature - m);
+    for (int i = lo; i < hi; ++i) part += expf(scaled(row[i], a.inv_temperature) - m);
     float denom;
     block_exclusive_scan_f(part, fscratch, &ftotal);
     denom = ftotal;
@@ -251,7 +256,7 @@ sample_kernel(float* __restrict__ logits, int V, long row_stride, SampleArgs a, 
                 const unsigned prefix = prefix_s;
                 const unsigned mask = pass == 0 ? 0u : (0xffffffffu << (shift + 8));
                 for (int i = tid; i < V; i += SAMPLE_THREADS) {
-                    const float z = row[i] * a.inv_temperature;
+                    const float z = scaled(row[i], a.inv_temperature);
                     const unsigned key = orderable(z);
                     if ((key & mask) != prefix) continue;
                     const float pr = expf(z - m) / denom;
@@ -288,14 +293,14 @@ sample_kernel(float* __restrict__ logits, int V, long row_stride, SampleArgs a, 
         int my_ties = 0;
         if (tie_keep != 0x7fffffff)
             for (int i = lo; i < hi; ++i) {
-                const float z = row[i] * a.inv_temperature;
+                const float z = scaled(row[i], a.inv_temperature);
                 if (orderable(z) == kth && expf(z - m) / denom >= thresh) ++my_ties;
             }
         int tie_rank = tie_keep != 0x7fffffff ? block_exclusive_scan(my_ties, iscratch, &itotal) : 0;
         __syncthreads();
         const int tie_rank0 = tie_rank;
         auto kept_prob = [&](int i, int& rank) -> float {
-            const float z = row[i] * a.inv_temperature;
+            const float z = scaled(row[i], a.inv_temperature);
             const float pr = expf(z - m) / denom;
             if (!(pr >= thresh)) return -1.f;
             const unsigned key = orderable(z);
@@ -342,7 +347,7 @@ sample_kernel(float* __restrict__ logits, int V, long row_stride, SampleArgs a, 
         const unsigned prefix = prefix_s;
         const unsigned mask = pass == 0 ? 0u : (0xffffffffu << (shift + 8));
         for (int i = tid; i < V; i += SAMPLE_THREADS) {
-            const unsigned key = orderable(row[i] * a.inv_temperature);
+            const unsigned key = orderable(scaled(row[i], a.inv_temperature));
             if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 0xff], 1);
         }
         __syncthreads();
@@ -364,7 +369,7 @@ sample_kernel(float* __restrict__ logits, int V, long row_stride, SampleArgs a, 
     __syncthreads();
     int my_ties = 0;
     for (int i = lo; i < hi; ++i) {
-        const float z = row[i] * a.inv_temperature;
+        const float z = scaled(row[i], a.inv_temperature);
         const unsigned key = orderable(z);
         if (key > kth) {
             const int slot = atomicAdd(&n_cand, 1);
@@ -380,7 +385,7 @@ sample_kernel(float* __restrict__ logits, int V, long row_stride, SampleArgs a, 
     {
         int rank = tie_rank;
         for (int i = lo; i < hi && rank < ties_needed; ++i) {
-            const float z = row[i] * a.inv_temperature;
+            const float z = scaled(row[i], a.inv_temperature);
             if (orderable(z) == kth) {
                 cand_z[n_above + rank] = z;
                 cand_id[n_above + rank] = i;
@@ -456,9 +461,9 @@ constexpr int SP_THREADS = 256;
 constexpr int SP_KMAX = 64;
 constexpr int SP_SORT = SP_PARTS * SP_KMAX;          // 2048 candidates
 
-// Larger for a larger logit (the two zeros are one), then for a lower id.
+// Larger for a larger logit, then for a lower id.
 __device__ __forceinline__ unsigned long long sp_key(float z, int id) {
-    return ((unsigned long long)orderable(__fadd_rn(z, 0.0f)) << 32) | (0xffffffffu - (unsigned)id);
+    return ((unsigned long long)orderable(z) << 32) | (0xffffffffu - (unsigned)id);
 }
 __device__ __forceinline__ float sp_logit(unsigned long long key) {
     const unsigned o = (unsigned)(key >> 32);
@@ -524,7 +529,7 @@ sample_parts_kernel(float* __restrict__ logits, int V, long row_stride, SampleAr
     float m = -INFINITY;
 #pragma unroll 8
     for (int i = tid; i < n; i += SP_THREADS) {
-        const float v = row[lo + i] * a.inv_temperature;
+        const float v = scaled(row[lo + i], a.inv_temperature);
         z[i] = v;
         m = fmaxf(m, v);
     }
