@@ -118,10 +118,9 @@ def test_gemm_generic(K, xd, wd, yd, M, N, K_):
 @pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("N,K_", [(130, 64), (33, 1000), (4100, 520), (31, 4), (256, 4096), (16500, 200), (20001, 36)])
 def test_few_tokens_in_float32_take_the_streaming_kernel_and_keep_the_order_of_the_sums(K, M, N, K_):
-    """Float operands with at most 32 tokens run a kernel of their own (32 weight rows a block, a thread per
-    row and token; 128 rows a block, every warp with rows of its own, from 16,384 rows on with at most 8
-    tokens).  It adds every output's products in ascending k like the tiled kernel, so the rows of a
-    step of few tokens equal, bit for bit, the same rows computed inside a step of many tokens."""
+    """Float operands with at most 32 tokens run a kernel that streams 16 to 128 weight rows a block.  It adds every
+    output's products in the order that K alone sets, so the rows of a step of few tokens equal, bit for bit, the same
+    rows computed inside a step of many tokens."""
     x, w, b = rnd((M, K_), torch.float32, seed=5), rnd((N, K_), torch.float32, seed=6), rnd((N,), torch.float32, seed=7)
     out = torch.full((M, N), 9.0, device=DEV)
     K.gemm_generic(x.to(DEV), w.to(DEV), out, bias=b.to(DEV))
@@ -143,10 +142,10 @@ def test_few_tokens_in_float32_take_the_streaming_kernel_and_keep_the_order_of_t
 
 @pytest.mark.parametrize("M,N,K_", [(97, 130, 64), (200, 257, 1000), (128, 128, 16), (300, 31, 4), (129, 640, 520)])
 def test_many_tokens_in_float32_take_the_large_tiles_and_keep_the_order_of_the_sums(K, M, N, K_):
-    """Float operands with more than 96 tokens run tiles of 128 x 128.  Every output is still one thread's sum in
-    ascending k: rows computed there equal, bit for bit, the same rows computed 70 at a time (the 64 x 64 tiles)
-    and 8 at a time (the streaming kernel); so do rows that accumulate and rows of wider buffers; unaligned rows
-    fall back to the small tiles and give the same bits."""
+    """Float operands with many tokens run tiles of 64 x 64 or 128 x 128.  The order of an output's additions is set by K
+    alone: rows computed there equal, bit for bit, the same rows computed 70 at a time and 8 at a time (the streaming
+    kernel); so do rows that accumulate and rows of wider buffers; unaligned rows take the kernel of any operands and give
+    the same bits."""
     x, w, b = rnd((M, K_), torch.float32, seed=15), rnd((N, K_), torch.float32, seed=16), rnd((N,), torch.float32, seed=17)
     out = torch.full((M, N), 9.0, device=DEV)
     K.gemm_generic(x.to(DEV), w.to(DEV), out, bias=b.to(DEV))
@@ -171,7 +170,9 @@ def test_many_tokens_in_float32_take_the_large_tiles_and_keep_the_order_of_the_s
     assert torch.equal(other, plain)
 
 
-@pytest.mark.parametrize("N,K_", [(65, 1024), (130, 1028), (64, 2052), (3, 8196), (200, 14336)])
+# fewer blocks of 64 rows than SMs (16 rows; 32 rows: 4096), about as many, two to four times as many (128 rows, few tokens)
+@pytest.mark.parametrize("N,K_", [(65, 1024), (130, 1028), (64, 2052), (3, 8196), (200, 14336), (4097, 516), (9601, 132),
+                                  (9602, 1028), (30001, 36)])
 def test_float32_sums_in_segments_of_k(K, N, K_):
     """Float operands: the K range is cut into at most eight segments whose sums are added in order, by the blocks of a
     cluster where rows start on 16-byte boundaries and by one block where they do not.  Every number of tokens (the

@@ -361,5 +361,16 @@ static inline int run_wait_selftest(int* err_word, int polls, int* seen, cudaStr
     return e == cudaSuccess ? 0 : (int)e;
 }
 
+// SMs of the device; asked once.
+static inline int sm_count() {
+    static int n = 0;
+    if (n == 0) {
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        n = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0 ? sms : 148;
+    }
+    return n;
+}
+
 }  // namespace tc
 }  // namespace zlm
