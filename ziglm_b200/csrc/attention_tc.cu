@@ -588,8 +588,10 @@ __device__ __forceinline__ void rotate_q_frags(uint32_t (&qf)[HD / 16][4], const
 }
 
 // MORE: the kernel also knows sinks, slopes and the norm of the heads (a form of its own, so that the plain one keeps its
-// registers).
-template <int HD, bool MORE>
+// registers).  STORE: it brings the step's new key and value itself (rope.store); the form without knows nothing of them
+// (64 sequences of 64 tokens, 16 heads of 128, rotation but no write: 16.7 us with one form for both, 14.9; 8 sequences of
+// 64, 32 heads of 64, neither: 4.0 and 3.5).
+template <int HD, bool MORE, bool STORE>
 __global__ void __launch_bounds__(ATC_THREADS, 2)
 attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                         AtcCommon a, FlatRope rope, const int* __restrict__ positions,
@@ -673,7 +675,7 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         int t = t0, kvh = kvh0, issued = 0;
         long vi = v0_item;
         bool alive = true;
-        bool waited = rope.fused && rope.store;      // the newest key and value are put in by this kernel itself
+        bool waited = STORE;                         // the newest key and value are put in by this kernel itself
         while (vi < g1 && t < T && alive) {
             const int p_t = pre[t + 1] - pre[t];
             // this block's pages of the item: the units [g0, g1) that fall on pages
@@ -755,27 +757,30 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         vi += p_t + IC;
         if (seg <= 0) continue;
         const int pos = positions[t];
+        const int seq = STORE ? seq_of_token[t] : 0;
         const int start = first_visible_key(pos, a.window);
         const int first_page = start / PAGE;
         // The new key and value, and the page they go to: asked for here, beside the queries, so that their latencies do
-        // not stand between the item's last page and its scores.  A thread takes element threadIdx.x (HD <= 128).
-        const bool brings_new = rope.fused && rope.store && j + seg == p_t && (int)threadIdx.x < HD;
+        // not stand between the item's last page and its scores.  A thread takes element threadIdx.x (HD <= 128).  The
+        // page's address needs the sequence's number: it is formed behind the queries' loads, which need not wait for it
+        // (64 sequences of 500 tokens, 8 key/value heads of 64: 18.5 -> 17.9 us).
+        const bool brings_new = STORE && j + seg == p_t && (int)threadIdx.x < HD;
         __nv_bfloat16 new_x = __float2bfloat16_rn(0.f), new_y = new_x, new_v = new_x;
         int new_page = 0;
         if (brings_new) {
             const int d = threadIdx.x;
             const __nv_bfloat16* knew = a.q + (long)t * a.q_row_stride + (long)(a.n_heads + kvh) * HD;
-            new_page = a.block_table[(long)seq_of_token[t] * a.bt_stride + first_page + p_t - 1];
             const int ii = d < half ? d : d < 2 * half ? d - half : d;
             new_x = knew[ii];
             if (d < 2 * half) new_y = knew[ii + half];
             new_v = ((MORE && rope.values_from_keys) ? knew : knew + (long)a.n_kv * HD)[d];
         }
-        if (half > 0 && t != t_angles) angles(t);
         const __nv_bfloat16* qrow = a.q + (long)t * a.q_row_stride + (long)kvh * group * HD;
         uint32_t qf[HD / 16][4];
         load_q_frags<HD>(qf, gid < group ? qrow + gid * HD : nullptr, gid + 8 < group ? qrow + (gid + 8) * HD : nullptr,
                          tid4);
+        if (brings_new) new_page = a.block_table[(long)seq * a.bt_stride + first_page + p_t - 1];   // waits for seq alone
+        if (half > 0 && t != t_angles) angles(t);
         if (half > 0) rotate_q_frags<HD>(qf, cs_s, sn_s, half, tid4);
         float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
         float slope2[2] = {0.f, 0.f};
@@ -802,7 +807,7 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
             const int s = it % C::STAGES;
             bool landed = warp_wait(full0 + 8 * s, (it / C::STAGES) & 1, abort_flag, a.err, ERR_ATT_FULL);
             const int p = first_page + j + i;
-            if (rope.fused && rope.store && j + i == p_t - 1) {
+            if (STORE && j + i == p_t - 1) {
                 // The page of position pos: its row pos % 64 is not in the cache yet.  The new key (rotated)
                 // and value go into the page in shared memory and into the cache, then everybody reads.
                 landed = !bar_consumers_or(!landed);
@@ -1301,7 +1306,7 @@ ZLM_EXPORT int zlm_attention_decode(const void* q, long q_row_stride, void* out,
 //   sinks, slopes   float [n_heads] or null, as zlm_attention_decode takes them
 //   scratch   floats for zlm_attention_decode_flat_scratch(...) of the same arguments
 namespace zlm {
-template <int HD, bool MORE>
+template <int HD, bool MORE, bool STORE>
 static int flat_blocks(int group, int T, int* smem_out) {
     const FlatSizes z = flat_sizes<HD>(group, T);
     if (smem_out) *smem_out = z.smem;
@@ -1312,11 +1317,11 @@ static int flat_blocks(int group, int T, int* smem_out) {
     if (max_dynamic == 0) {
         // the kernel's static shared memory counts against the same 227 KB
         cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, attn_decode_flat_kernel<HD, MORE>) != cudaSuccess) { cudaGetLastError(); return 0; }
+        if (cudaFuncGetAttributes(&fa, attn_decode_flat_kernel<HD, MORE, STORE>) != cudaSuccess) { cudaGetLastError(); return 0; }
         const int room = 227 * 1024 - (int)fa.sharedSizeBytes;
-        if (cudaFuncSetAttribute(attn_decode_flat_kernel<HD, MORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, room) !=
+        if (cudaFuncSetAttribute(attn_decode_flat_kernel<HD, MORE, STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, room) !=
                 cudaSuccess ||
-            cudaFuncSetAttribute(attn_decode_flat_kernel<HD, MORE>, cudaFuncAttributePreferredSharedMemoryCarveout,
+            cudaFuncSetAttribute(attn_decode_flat_kernel<HD, MORE, STORE>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared) != cudaSuccess) {
             cudaGetLastError();
             return 0;
@@ -1324,16 +1329,24 @@ static int flat_blocks(int group, int T, int* smem_out) {
         max_dynamic = room;
     }
     if (z.smem > max_dynamic) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_flat_kernel<HD, MORE>, ATC_THREADS, z.smem) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_flat_kernel<HD, MORE, STORE>, ATC_THREADS, z.smem) !=
         cudaSuccess) return 0;
     return sms * min(per_sm, 2);
+}
+
+typedef void (*FlatKernel)(const CUtensorMap, const CUtensorMap, AtcCommon, FlatRope, const int*, const int*, int, int*, float*,
+                           __nv_bfloat16*);
+template <int HD, bool MORE, bool STORE>
+static int flat_form(int group, int T, int* smem_out, FlatKernel* kernel) {
+    *kernel = attn_decode_flat_kernel<HD, MORE, STORE>;
+    return flat_blocks<HD, MORE, STORE>(group, T, smem_out);
 }
 }  // namespace zlm
 
 ZLM_EXPORT int zlm_attention_decode_flat_blocks(int T, int n_heads, int n_kv, int hd) {
     if (T <= 0 || T > FLAT_MAX_TOKENS || n_heads <= 0 || n_kv <= 0 || n_heads % n_kv || n_heads / n_kv > 16) return 0;
-    if (hd == 128) return flat_blocks<128, false>(n_heads / n_kv, T, nullptr);
-    if (hd == 64) return flat_blocks<64, false>(n_heads / n_kv, T, nullptr);
+    if (hd == 128) return flat_blocks<128, false, true>(n_heads / n_kv, T, nullptr);
+    if (hd == 64) return flat_blocks<64, false, true>(n_heads / n_kv, T, nullptr);
     return 0;
 }
 
@@ -1386,14 +1399,16 @@ ZLM_EXPORT int zlm_attention_decode_flat(const void* q, long q_row_stride, void*
     a.slopes = slopes;
     const int group = n_heads / n_kv;
     int smem = 0;
-    const int resident = more ? (hd == 128 ? flat_blocks<128, true>(group, T, &smem) : flat_blocks<64, true>(group, T, &smem))
-                              : (hd == 128 ? flat_blocks<128, false>(group, T, &smem) : flat_blocks<64, false>(group, T, &smem));
+    FlatKernel kern = nullptr;
+    const int resident =
+        rope.store ? (more ? (hd == 128 ? flat_form<128, true, true>(group, T, &smem, &kern) : flat_form<64, true, true>(group, T, &smem, &kern))
+                           : (hd == 128 ? flat_form<128, false, true>(group, T, &smem, &kern) : flat_form<64, false, true>(group, T, &smem, &kern)))
+                   : (more ? (hd == 128 ? flat_form<128, true, false>(group, T, &smem, &kern) : flat_form<64, true, false>(group, T, &smem, &kern))
+                           : (hd == 128 ? flat_form<128, false, false>(group, T, &smem, &kern) : flat_form<64, false, false>(group, T, &smem, &kern)));
     if (resident <= 0) return ZLM_ERR_UNSUPPORTED;
     if (n_blocks <= 0) n_blocks = resident;
     if (!counters || !scratch || zlm_attention_decode_flat_scratch(T, n_heads, n_kv, hd, n_blocks) > scratch_floats)
         return ZLM_ERR_BAD_ARG;
-    auto* kern = more ? (hd == 128 ? attn_decode_flat_kernel<128, true> : attn_decode_flat_kernel<64, true>)
-                      : (hd == 128 ? attn_decode_flat_kernel<128, false> : attn_decode_flat_kernel<64, false>);
     cudaError_t e = launch_pdl(kern, dim3(n_blocks), dim3(ATC_THREADS), (size_t)smem, stream, mk, mv, a, rope, positions,
                                seq_of_token, T, counters, scratch, (__nv_bfloat16*)out);
     if (e != cudaSuccess) return (int)e;
