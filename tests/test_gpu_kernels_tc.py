@@ -56,9 +56,11 @@ def test_gemm_tc_split_k_is_exact_in_order(K, splits, T):
 
 
 # Split launches by stage count: four stages (4 K blocks a part and fewer), five or six (one block an SM, 5 and more K
-# blocks a part), a last part that is shorter, more tiles than are split; and the first sizes of the wider tiles.
+# blocks a part), a last part that is shorter, six parts (60 tiles of 16 tokens), two parts of more tiles than SMs, more
+# tiles than are split; and the first sizes of the wider tiles.
 @pytest.mark.parametrize("T", [1, 16, 17, 32, 64, 65, 128])
-@pytest.mark.parametrize("N,K_", [(256, 2048), (384, 2560), (2048, 8192), (1000, 1096), (28416, 512), (28544, 512)])
+@pytest.mark.parametrize("N,K_", [(256, 2048), (384, 2560), (2048, 8192), (1000, 1096), (7680, 2048), (28416, 512), (28416, 2048),
+                                  (28544, 512)])
 def test_gemm_tc_split_stages(K, T, N, K_):
     x, w, b = rnd((T, K_), BF, seed=51).to(DEV), rnd((N, K_), BF, 0.05, seed=52).to(DEV), rnd((N,), BF, seed=53).to(DEV)
     base = rnd((T, N), torch.float32, seed=54).to(DEV)
@@ -75,7 +77,12 @@ def test_gemm_tc_split_stages(K, T, N, K_):
         # the norm rides on the sum: x * gain and the sums of squares come from the residual the launch leaves
         gain, hb = rnd((N,), torch.float32, seed=55).to(DEV), torch.empty(T, N, dtype=BF, device=DEV)
         ssq, res = torch.zeros(T, -(-N // 128), device=DEV), base.clone()
-        if K.gemm_tc(x, w, res, accumulate=True, norm_out=(gain, 0.0, hb, ssq)) == 2:
+        fused = K.gemm_tc(x, w, res, accumulate=True, norm_out=(gain, 0.0, hb, ssq))
+        # more tiles than SMs are split only where two blocks of each fit the device and K is long for the tokens; no split,
+        # no norm
+        tiles = -(-N // 128)
+        assert fused == (2 if tiles <= 148 or (T <= 16 and tiles <= 222 and (T <= 4 or K_ >= 2048)) else 1)
+        if fused == 2:
             assert torch.equal(hb, (res * gain).to(BF))
             assert torch.allclose(ssq.sum(1), (res * res).sum(1), rtol=N * 2.0 ** -23)
         assert ((res.double() - (want + base.double())).abs() <= bound).all()

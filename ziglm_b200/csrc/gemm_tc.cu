@@ -931,7 +931,7 @@ template <int BN, int MODE>
 static int launch_split(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& my, const TcArgs& a, cudaStream_t s) {
     // two of the deep form still fit an SM: a cluster of eight finds its SMs in one part of the chip
     constexpr int DEEP = BN == 16 ? SPLIT_K + 6 : SPLIT_K + 5;
-    if (a.grid_x * a.splits <= 148 && a.kb_per_split > 4) return launch_tc<BN, MODE, DEEP>(mw, mx, my, a, s);
+    if (a.grid_x * a.splits <= sm_count() && a.kb_per_split > 4) return launch_tc<BN, MODE, DEEP>(mw, mx, my, a, s);
     return launch_tc<BN, MODE, SPLIT_K + 4>(mw, mx, my, a, s);
 }
 
@@ -953,10 +953,10 @@ static int pick_mode(int mode, const CUtensorMap& mw, const CUtensorMap& mx, con
         case OUT_F32: return launch_tc<BN, OUT_F32>(mw, mx, my, a, s);
         case OUT_F32_ACC: return launch_tc<BN, OUT_F32_ACC>(mw, mx, my, a, s);
         case OUT_BF16_GLU:
-            if (BN <= 32 && a.splits == 1 && a.grid_x <= 2 * 148) return launch_tc<BN, OUT_BF16_GLU, 4>(mw, mx, my, a, s);
+            if (BN <= 32 && a.splits == 1 && a.grid_x <= 2 * sm_count()) return launch_tc<BN, OUT_BF16_GLU, 4>(mw, mx, my, a, s);
             return launch_tc<BN, OUT_BF16_GLU>(mw, mx, my, a, s);
         case OUT_BF16_GEGLU:
-            if (BN <= 32 && a.splits == 1 && a.grid_x <= 2 * 148) return launch_tc<BN, OUT_BF16_GEGLU, 4>(mw, mx, my, a, s);
+            if (BN <= 32 && a.splits == 1 && a.grid_x <= 2 * sm_count()) return launch_tc<BN, OUT_BF16_GEGLU, 4>(mw, mx, my, a, s);
             return launch_tc<BN, OUT_BF16_GEGLU>(mw, mx, my, a, s);
         default: return launch_tc<BN, OUT_BF16>(mw, mx, my, a, s);
     }
@@ -1083,17 +1083,23 @@ static int gemm_tc_run(const void* X, const void* W, const void* bias, int bias_
     int s = splits;
     if (s == 0) {
         s = 1;
-        // As many blocks as are resident at once: three an SM with tiles of 16 tokens, two with wider ones; more start
-        // late and cost more than they bring (16 tokens: 16384 x 2048 gated, 128 tiles, in three parts 13.7 us, in two
-        // 16.1; 27648 x 5120 gated, 216 tiles, in two 45.1, whole 47.4; 28672 x 4096 gated, 224 tiles, whole 40.5, in
-        // two 44.2).  From 32 tokens on a rank's share of the reduction over the cluster grows with the tile, and a
-        // product that stores does best short of that (6144 x 4096, 64 tokens: five ranks 13.5 us, six 19.7).
+        // As many parts as let every cluster be resident at once: three blocks an SM with tiles of 16 tokens, two with
+        // wider ones.  A cluster lies within one of the chip's groups of SMs, and what a group has left over stays empty:
+        // clusters of seven and eight blocks found room for 384 and 385 blocks of 444 (256 and 259 of 296), of three to
+        // six for 410 to 420 (270 to 284), pairs for all.  One part more and the clusters that do not fit run after the
+        // others (K = 4096; 16 tokens, 60 tiles: six parts 12.8 us, seven 17.8; 32 tokens: 40 tiles in six 10.5, in seven
+        // 16.0; 48 in five 12.1, in six 17.6; 96 in two 24.0, in three 32.0).
         if (bn <= 64) {
-            const int blocks = bn == 16 ? 3 * 148 : (glu || accumulate) ? 2 * 148 : 240;
-            s = blocks / tiles;
-            if (s < 1) s = 1;
-            if (s > 8) s = 8;
-            const int most = a.kb_total / 4 > 0 ? a.kb_total / 4 : 1;   // at least 4 K blocks per CTA
+            const long blocks = (bn == 16 ? 3L : 2L) * sm_count();
+            s = 8;
+            while (s > 1 && (long)tiles * s > (s > 6 ? blocks * 32 / 37 : s > 2 ? blocks * 10 / 11 : blocks)) --s;
+            // Four K blocks a part at least; more where the tiles alone give (nearly) every SM a block and a second part
+            // is hardly worth its reduction (K = 512: 16 tokens, 222 tiles, 9.1 us in two parts, 7.3 whole; 33 tokens,
+            // 147 tiles stored, 10.1 and 8.2).
+            int least = 4;
+            if (bn == 16 && T > 4 && 5 * tiles > 6 * sm_count()) least = 16;
+            if (bn > 16 && !glu && !accumulate && 5 * tiles > 4 * sm_count()) least = 8;
+            const int most = a.kb_total / least > 0 ? a.kb_total / least : 1;
             if (s > most) s = most;
         }
     }
@@ -1107,15 +1113,8 @@ static int gemm_tc_run(const void* X, const void* W, const void* bias, int bias_
         *norm_fused = 1;
     }
     // one tile per block when K is split; otherwise as many blocks as fit the GPU share the tiles
-    static int sm_count = 0;
-    if (sm_count == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0)
-            sm_count = 148;
-    }
-    const int per_sm = bn <= 64 ? 2 : 1;
-    a.grid_x = (s > 1 || tiles < sm_count * per_sm) ? tiles : sm_count * per_sm;
+    const int room = sm_count() * (bn <= 64 ? 2 : 1);
+    a.grid_x = (s > 1 || tiles < room) ? tiles : room;
     CUtensorMap mw, mx, my;
     int rc = cached_map(&mw, W, N, K, ldw, TC_BM);
     if (rc) return rc;
