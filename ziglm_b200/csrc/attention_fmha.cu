@@ -474,7 +474,7 @@ fmha_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             const int lo_vis = max(start, key0) - key0, hi_vis = min(pos, key_end) - key0, keep_vis = keep - key0;
             // One reading of the row: the loads of all its scores are issued together and waited for once
             // (a tcgen05.ld and its wait cost about as much as the arithmetic on 32 scores), the row stays in
-            // registers between the maximum and the exponentials, and the stores of P are waited for once.
+            // registers between the maximum and the exponentials, and the stores of P are waited for once a page.
             const float bias0 = slope * (float)(key0 - pos);
             const uint32_t p_bar = p_full0 + 8 * FM_NP * t;
             if (np == FM_NP)
