@@ -92,9 +92,9 @@ constexpr int SPLIT_K = 100;
 template <int BN, int DEEP = 0> struct TcCfg {
     // Narrow tiles (decode steps) keep few stages, so that three or four blocks fit an SM: the blocks of
     // the next product become resident while this one drains and request their weight tiles early.
-    // DEEP: the gated product of a decode step runs as one tile of a megabyte of weights per block, at
-    // most two blocks per SM; what bounds it is the bytes each block has in flight, so it takes a fourth
-    // stage (measured: five and more cost the next product its early residence).
+    // DEEP: the gated product of a decode step, and any whole product of more tiles than SMs, runs as one tile of a
+    // megabyte of weights per block, at most two blocks per SM; what bounds it is the bytes each block has in flight, so
+    // it takes a fourth stage (measured: five and more cost the next product its early residence).
     // A product whose K is split takes four stages in the same room (no staging area), and five or six where there is at
     // most one block an SM and more K blocks than four: a small product's weights (four K blocks a block) are then all
     // requested before the kernel before it ends, and a lone block has enough bytes in flight for its SM's share of
@@ -951,15 +951,30 @@ static int pick_mode(int mode, const CUtensorMap& mw, const CUtensorMap& mx, con
             }
         }
     }
+    if constexpr (BN <= 32) {
+        // At most two blocks an SM: the fourth stage's room is there.  Gated products take it at any size, the others from
+        // more than one block an SM on: with three stages a third block of theirs fits, and the next product's blocks lie
+        // unevenly (K = 4096, 240 tiles: 1 token 46.1 -> 41.3 us, 16 tokens 47.2 -> 42.0).
+        if (a.grid_x <= 2 * sm_count()) {
+            switch (mode) {
+                case OUT_BF16_GLU: return launch_tc<BN, OUT_BF16_GLU, 4>(mw, mx, my, a, s);
+                case OUT_BF16_GEGLU: return launch_tc<BN, OUT_BF16_GEGLU, 4>(mw, mx, my, a, s);
+                default: break;
+            }
+            if (a.grid_x > sm_count()) {
+                switch (mode) {
+                    case OUT_F32: return launch_tc<BN, OUT_F32, 4>(mw, mx, my, a, s);
+                    case OUT_F32_ACC: return launch_tc<BN, OUT_F32_ACC, 4>(mw, mx, my, a, s);
+                    default: return launch_tc<BN, OUT_BF16, 4>(mw, mx, my, a, s);
+                }
+            }
+        }
+    }
     switch (mode) {
         case OUT_F32: return launch_tc<BN, OUT_F32>(mw, mx, my, a, s);
         case OUT_F32_ACC: return launch_tc<BN, OUT_F32_ACC>(mw, mx, my, a, s);
-        case OUT_BF16_GLU:
-            if (BN <= 32 && a.splits == 1 && a.grid_x <= 2 * sm_count()) return launch_tc<BN, OUT_BF16_GLU, 4>(mw, mx, my, a, s);
-            return launch_tc<BN, OUT_BF16_GLU>(mw, mx, my, a, s);
-        case OUT_BF16_GEGLU:
-            if (BN <= 32 && a.splits == 1 && a.grid_x <= 2 * sm_count()) return launch_tc<BN, OUT_BF16_GEGLU, 4>(mw, mx, my, a, s);
-            return launch_tc<BN, OUT_BF16_GEGLU>(mw, mx, my, a, s);
+        case OUT_BF16_GLU: return launch_tc<BN, OUT_BF16_GLU>(mw, mx, my, a, s);
+        case OUT_BF16_GEGLU: return launch_tc<BN, OUT_BF16_GEGLU>(mw, mx, my, a, s);
         default: return launch_tc<BN, OUT_BF16>(mw, mx, my, a, s);
     }
 }
