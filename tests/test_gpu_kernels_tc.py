@@ -2,6 +2,7 @@
 steps) against plain float32 statements of the same operations, at sizes other than the engine's."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -250,6 +251,32 @@ def test_attention_decode_flat_by_a_cluster_an_item(K, hd, seqs, longest):
     assert torch.allclose(got, want, atol=2e-2, rtol=2e-2)
     flat, _ = run_decode_flat(K, 32, 8, hd, lens, None, 290, seed=41)      # not a whole wave: no clusters
     assert torch.allclose(got, flat, atol=1e-2, rtol=1e-2)
+
+
+# 1.5 + 2^-8 lies halfway between two bf16 numbers; formed as (n (1.5 + 2^-8)) (1 / n) it is above that for these n
+HALFWAY = 1.5 + 2.0 ** -8
+HALFWAY_KEYS = [n for n in range(2, 65, 2) if np.float32(n * HALFWAY) * (np.float32(1.0) / np.float32(n)) > np.float32(HALFWAY)]
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("seqs", [1, 64])
+def test_attention_decode_flat_rounds_the_quotient_once(K, hd, seqs):
+    """An item of one page, by one block (64 sequences) and by a cluster of blocks (one sequence): half of the values are
+    1.5, half 1.5 + 2^-7, every score is 0.  The sums and their number are exact, the quotient is a tie that goes to 1.5."""
+    assert HALFWAY_KEYS == [14, 28, 30, 56, 60]
+    nh, nkv = 32, 8
+    for n in HALFWAY_KEYS:
+        v = torch.full((seqs, nkv, 64, hd), 1.5, dtype=BF)
+        v[:, :, 1:n:2] = 1.5 + 2.0 ** -7
+        out = torch.zeros(seqs, nh * hd, dtype=BF, device=DEV)
+        n_blocks = K.attention_decode_flat_blocks(seqs, nh, nkv, hd)
+        scratch = torch.empty(K.attention_decode_flat_scratch(seqs, nh, nkv, hd, n_blocks), device=DEV)
+        ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+        assert K.attention_decode_flat(torch.zeros(seqs, nh * hd, dtype=BF, device=DEV), out, nh, nkv, hd, 1.0, None,
+                                       ints([n - 1] * seqs), ints(list(range(seqs))), ints([[i] for i in range(seqs)]),
+                                       torch.zeros_like(v).to(DEV), v.to(DEV), 64, n_blocks,
+                                       torch.zeros(seqs * nkv, dtype=torch.int32, device=DEV), scratch)
+        assert (out == 1.5).all(), n
 
 
 def test_attention_decode_flat_many_tokens(K):

@@ -612,18 +612,23 @@ __device__ __forceinline__ void rotate_q_frags(uint32_t (&qf)[HD / 16][4], const
     }
 }
 
-// Four neighbouring sums over their denominator, times the gate, to the outputs.
-__device__ __forceinline__ void store_quad(const float4& acc, float inv, const __nv_bfloat16* grow, int f, __nv_bfloat16* orow) {
-    float y[4] = {acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv};
-    if (grow != nullptr) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) y[i] *= gate_factor(grow, 4 * f + i);
-    }
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[1]), hi = __floats2bfloat162_rn(y[2], y[3]);
+// Four neighbouring outputs, rounded.
+__device__ __forceinline__ void store_quad(float x, float y, float z, float w, int f, __nv_bfloat16* orow) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(x, y), hi = __floats2bfloat162_rn(z, w);
     uint2 packed;
     packed.x = *reinterpret_cast<const uint32_t*>(&lo);
     packed.y = *reinterpret_cast<const uint32_t*>(&hi);
     *reinterpret_cast<uint2*>(orow + 4 * f) = packed;
+}
+// Four neighbouring sums over their denominator, times the gate, to the outputs.  The quotient is rounded once: a product
+// with 1 / den, rounded twice, sends quotients halfway between two bf16 numbers to the wrong one of them.
+__device__ __forceinline__ void store_quad(const float4& acc, float den, const __nv_bfloat16* grow, int f, __nv_bfloat16* orow) {
+    float y[4] = {acc.x / den, acc.y / den, acc.z / den, acc.w / den};
+    if (grow != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] *= gate_factor(grow, 4 * f + i);
+    }
+    store_quad(y[0], y[1], y[2], y[3], f, orow);
 }
 
 // MORE: the kernel also knows sinks, slopes and the norm of the heads (a form of its own, so that the plain one keeps its
@@ -958,7 +963,7 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                     den += ml[w * 16 + r] * wgt;
                 }
                 if (pieces == 1 && !own_item) {
-                    store_quad(acc, 1.f / den, grow, f, orow);
+                    store_quad(acc, den, grow, f, orow);
                 } else {
                     *reinterpret_cast<float4*>(slot + 4 * f) = acc;
                     if (d == 0) { slot[group * HD + 2 * r] = big; slot[group * HD + 2 * r + 1] = den; }
@@ -992,7 +997,7 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                     v.x += __shfl_xor_sync(0xffffffffu, v.x, o); v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
                     v.z += __shfl_xor_sync(0xffffffffu, v.z, o); v.w += __shfl_xor_sync(0xffffffffu, v.w, o);
                 }
-                if (u == 0 && f < quads) store_quad(v, 1.f / den, grow, f, orow);
+                if (u == 0 && f < quads) store_quad(v, den, grow, f, orow);
             }
             cluster_sync_arrive_wait();            // the others may still read this block's piece
             break;
@@ -1038,7 +1043,9 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                             den += ml2[u].y * w;
                             acc.x += v[u].x * w; acc.y += v[u].y * w; acc.z += v[u].z * w; acc.w += v[u].w * w;
                         }
-                        store_quad(acc, 1.f / den, grow, f, orow);
+                        const float inv = 1.f / den;
+                        store_quad(acc.x * (inv * gate_factor(grow, 4 * f)), acc.y * (inv * gate_factor(grow, 4 * f + 1)),
+                                   acc.z * (inv * gate_factor(grow, 4 * f + 2)), acc.w * (inv * gate_factor(grow, 4 * f + 3)), f, orow);
                     }
                 } else if (pieces <= 2 * HD) {
                     // (m, l) of every piece in one round of loads, turned into weights 2^(m - M) / L in place
@@ -1087,11 +1094,7 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                         }
                         acc.x *= gate_factor(grow, 4 * f); acc.y *= gate_factor(grow, 4 * f + 1);
                         acc.z *= gate_factor(grow, 4 * f + 2); acc.w *= gate_factor(grow, 4 * f + 3);
-                        __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
-                        uint2 packed;
-                        packed.x = *reinterpret_cast<uint32_t*>(&lo);
-                        packed.y = *reinterpret_cast<uint32_t*>(&hi);
-                        *reinterpret_cast<uint2*>(orow + 4 * f) = packed;
+                        store_quad(acc.x, acc.y, acc.z, acc.w, f, orow);
                     }
                 } else {
                     // more pieces than the merge area holds weights for: straight from global memory
