@@ -241,11 +241,15 @@ def test_attention_decode_flat_many_short_sequences(K, hd, n_blocks):
 
 
 @pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("seqs", [1, 4, 5, 9, 18, 19])
+@pytest.mark.parametrize("seqs", [1, 2, 3, 4, 5, 9, 18, 19])
 @pytest.mark.parametrize("longest", [3, 64, 520, 1500])
 def test_attention_decode_flat_by_a_cluster_an_item(K, hd, seqs, longest):
-    """Steps of few items take clusters of 8, 4 or 2 blocks, an item each where no item is much longer than the others
-    (fewer pages than blocks, shares that do not come out even), else the flat division; more items take none."""
+    """Steps of few items take clusters of 8 blocks, an item each where no item is much longer than the others (fewer pages
+    than blocks, shares that do not come out even), else the flat division; more items take none: what clusters of 4 and
+    of 2 won for equal sequences unequal ones lost."""
+    blocks = K.attention_decode_flat_blocks(seqs, 32, 8, hd)
+    assert K.attention_decode_flat_cluster(seqs, 32, 8, hd) == (8 if seqs * 8 * 12 <= blocks else 1)
+    assert (seqs <= 3) == (seqs * 8 * 12 <= blocks)                        # of 148 SMs
     lens = [longest * (1 + i % 5) // 5 for i in range(seqs)]
     got, want = run_decode_flat(K, 32, 8, hd, lens, None, 0, seed=41)
     assert torch.allclose(got, want, atol=2e-2, rtol=2e-2)

@@ -481,11 +481,10 @@ __device__ __forceinline__ float gate_factor(const __nv_bfloat16* g, long i) {
 // A block that holds many item starts thereby gets fewer pages.  Page k of item i is the unit
 // V_i + item_cost + k, with V_i the units before the item; block c owns the units [c * chunk, (c + 1) * chunk).
 //
-// A step of few items is launched in clusters of as many blocks as the items leave for each.  If no item is so long that its
-// cluster would take longer than the blocks of the flat division and their merge, a cluster takes an item: its blocks take
-// equal shares of the pages, leave their pieces in shared memory, meet at the cluster's barrier and merge a share of the
-// result each.  That replaces a trip of every piece through global memory, a fence and a counter (2.7 of 8.7 us where
-// there is little else to do).
+// A step of few items (flat_cluster) is launched in clusters of eight blocks.  If no item is so long that its cluster would
+// take longer than the blocks of the flat division and their merge, a cluster takes an item: its blocks take equal shares of
+// the pages, leave their pieces in shared memory, meet at the cluster's barrier and merge a share of the result each.  That
+// replaces a trip of every piece through global memory, a fence and a counter (2.7 of 8.7 us where there is little else to do).
 constexpr int FLAT_MAX_TOKENS = 4096;
 // pages a block may have more than the flat division gives it before a cluster an item takes longer
 template <int HD> __host__ __device__ constexpr int merge_cost() { return 512 / HD; }
@@ -1424,15 +1423,27 @@ static int flat_blocks(int group, int T, int* smem_out) {
 
 typedef void (*FlatKernel)(const CUtensorMap, const CUtensorMap, AtcCommon, FlatRope, const int*, const int*, int, int*, float*,
                            __nv_bfloat16*);
-// Clusters of c blocks that are resident at once, with the shared memory of the call; asked once for each size of it.
-static int flat_clusters(FlatKernel kern, int c, int smem, int resident) {
-    struct Known { FlatKernel kern; int c, smem, n; };
+// The steps launched in clusters: eight blocks an item leave a third of the resident ones over.  A cluster finds its place
+// later than eight blocks by themselves do, and a launch of clusters has 256 of 296 blocks: a step whose items are too
+// unequal or too long for a cluster each pays for that.  Microseconds a layer, clusters of eight against none (8 key/value
+// heads of 128 and of 64): one sequence of 130 / 1,000 / 4,096 / 8,000 tokens -1.2 / -4.4 / -1.0 / 0.0 and -1.2 / -4.1 / -4.3 /
+// -0.2, three of 4,096 / 300 to 4,000 / 300 to 8,000 -4.0 / -2.5 / +0.9 and -2.1 / -1.7 / -0.9; four sequences
+// (32 items) +0.6 / 0.0 / -2.6 and +1.0 / +0.5 / -1.6 at 130 / 1,000 / 4,096 tokens; six and eight in clusters of four +1.4 /
+// +0.2 / +0.7, +1.4 / -0.3 / -2.1 and, 300 to 8,000 tokens, +1.6 and +0.8, more where the memory is the bound (eight of 300
+// to 8,000 at heads of 64, sixteen layers: 3.6 percent of the step); eight to sixteen items of one key/value head -0.5 to -2.6.
+constexpr int FLAT_CLUSTER = 8;
+static bool flat_few_items(long items, int resident) { return items * FLAT_CLUSTER * 3 <= 2L * resident; }
+
+// Clusters of FLAT_CLUSTER blocks that are resident at once, with the shared memory of the call; asked once for each size of it.
+static int flat_clusters(FlatKernel kern, int smem, int resident) {
+    constexpr int c = FLAT_CLUSTER;
+    struct Known { FlatKernel kern; int smem, n; };
     static std::mutex mu;
     static Known known[64];
     static int used = 0;
     std::lock_guard<std::mutex> lock(mu);
     for (int i = 0; i < used; ++i)
-        if (known[i].kern == kern && known[i].c == c && known[i].smem == smem) return known[i].n;
+        if (known[i].kern == kern && known[i].smem == smem) return known[i].n;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(resident / c * c);
     cfg.blockDim = dim3(ATC_THREADS);
@@ -1447,7 +1458,7 @@ static int flat_clusters(FlatKernel kern, int c, int smem, int resident) {
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
     n = min(n, resident / c);
-    if (used < 64) known[used++] = {kern, c, smem, n};
+    if (used < 64) known[used++] = {kern, smem, n};
     return n;
 }
 
@@ -1471,6 +1482,12 @@ ZLM_EXPORT long zlm_attention_decode_flat_scratch(int T, int n_heads, int n_kv, 
     if (T <= 0 || n_kv <= 0 || n_heads <= 0 || n_blocks <= 0) return 0;
     const long slot = ((long)(n_heads / n_kv) * (hd + 2) + 3) / 4 * 4;
     return ((long)n_blocks + (long)T * n_kv) * slot;
+}
+
+// Blocks a cluster of such a step's launch with one resident wave (1: none), 0: sizes the kernel refuses.
+ZLM_EXPORT int zlm_attention_decode_flat_cluster(int T, int n_heads, int n_kv, int hd) {
+    const int resident = zlm_attention_decode_flat_blocks(T, n_heads, n_kv, hd);
+    return resident <= 0 ? 0 : flat_few_items((long)T * n_kv, resident) ? FLAT_CLUSTER : 1;
 }
 
 ZLM_EXPORT int zlm_attention_decode_flat(const void* q, long q_row_stride, void* out, int T, int n_heads, int n_kv,
@@ -1524,16 +1541,11 @@ ZLM_EXPORT int zlm_attention_decode_flat(const void* q, long q_row_stride, void*
     if (n_blocks <= 0) n_blocks = resident;
     if (!counters || !scratch || zlm_attention_decode_flat_scratch(T, n_heads, n_kv, hd, n_blocks) > scratch_floats)
         return ZLM_ERR_BAD_ARG;
-    // Clusters of the most blocks with which every item finds its cluster resident.  Clusters of eight and four do not fill
-    // every group of SMs (256 and some 270 of 296 blocks): a step that keeps to the flat division all the same has that
-    // many blocks fewer, and the same bytes in flight as the memory needs.
     int cl = 1;
-    if (n_blocks == resident)
-        for (int c = 8; c > 1 && cl == 1; c /= 2)
-            if ((long)T * n_kv * c <= resident) {
-                const int n = flat_clusters(kern, c, smem, resident);
-                if ((long)T * n_kv <= n) { cl = c; n_blocks = n * c; }
-            }
+    if (n_blocks == resident && flat_few_items((long)T * n_kv, resident)) {
+        const int n = flat_clusters(kern, smem, resident);
+        if ((long)T * n_kv <= n) { cl = FLAT_CLUSTER; n_blocks = n * cl; }
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_blocks);
     cfg.blockDim = dim3(ATC_THREADS);

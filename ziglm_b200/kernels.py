@@ -170,6 +170,7 @@ _PROTOTYPES = {
                                       c_void_p, c_long, c_int, c_int, c_int, c_void_p, c_int, c_float, c_void_p, c_void_p,
                                       c_int, c_void_p, c_void_p, c_void_p, c_long, c_void_p],
         "zlm_attention_decode_flat_blocks": [c_int, c_int, c_int, c_int],
+        "zlm_attention_decode_flat_cluster": [c_int, c_int, c_int, c_int],
         "zlm_attention_decode_flat_scratch": [c_int, c_int, c_int, c_int, c_int],
         "zlm_attention_prefill": [c_void_p, c_long, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int,
                                   c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_long, c_int, c_void_p],
@@ -1483,6 +1484,11 @@ def _gate_args(gate: Optional[torch.Tensor], n_rows: int, width: int):
 def attention_decode_flat_blocks(n_tokens: int, n_heads: int, n_kv: int, head_dim: int) -> int:
     """Blocks of one resident wave of the flat decode kernel for a step of ``n_tokens`` (0: sizes it refuses)."""
     return int(_fn("attention_tc", "zlm_attention_decode_flat_blocks")(n_tokens, n_heads, n_kv, head_dim))
+
+
+def attention_decode_flat_cluster(n_tokens: int, n_heads: int, n_kv: int, head_dim: int) -> int:
+    """Blocks of a cluster in which such a step is launched with one resident wave (1: no clusters, 0: sizes it refuses)."""
+    return int(_fn("attention_tc", "zlm_attention_decode_flat_cluster")(n_tokens, n_heads, n_kv, head_dim))
 
 
 def attention_decode_flat_scratch(n_tokens: int, n_heads: int, n_kv: int, head_dim: int, n_blocks: int) -> int:
