@@ -73,6 +73,22 @@ def test_byte_and_flop_counts():
 import pytest
 
 
+def test_a_wait_error_of_a_library_that_the_line_does_not_list_ends_the_run():
+    sys.path.insert(0, ROOT)
+    import bench
+
+    class Kernels:
+        codes = {"gemm_tc": 0, "attention_tc": 3, "gemm_generic": 0}
+        wait_errors = classmethod(lambda cls: dict(cls.codes))
+        describe_wait_errors = staticmethod(lambda codes: ", ".join(codes))
+
+    assert bench.wait_errors(Kernels) == [0, 3, 0]
+    Kernels.codes["gemm_generic"] = 2
+    with pytest.raises(RuntimeError, match="gemm_generic"):
+        bench.wait_errors(Kernels)
+    assert bench.wait_errors(Kernels, ("gemm_generic", "gemm_tc", "attention_tc")) == [2, 0, 3]
+
+
 @pytest.mark.gpu
 def test_the_line_of_a_shallow_run_has_every_key_of_the_contract():
     """`bench.py` on two layers of the benchmarked shape: one JSON line with the metric, the end-to-end figure and
