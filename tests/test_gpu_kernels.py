@@ -233,6 +233,26 @@ def test_float32_products_at_the_ends_of_the_range(K, M):
     assert torch.equal(out, x[:, :N])
 
 
+@pytest.mark.parametrize("wide", [True, False])
+@pytest.mark.parametrize("M", [1, 40, 200])
+def test_float32_products_with_weights_from_the_kernel_before(K, wide, M):
+    """The weights are what the launch just before writes (it lets the next kernel start early): many rows, so that it is at
+    work for long, in rows on 16-byte boundaries (TMA) and off them."""
+    N, K_ = 20000, 512
+    x = rnd((M, K_), torch.float32, seed=51).to(DEV)
+    w16 = rnd((N, K_), torch.bfloat16, seed=52).to(DEV)
+    buf = torch.empty(N, K_ + (4 if wide else 1), device=DEV)
+    w = buf[:, :K_]
+    out, want = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    K.gemm_generic(x, w16.float(), want)
+    for _ in range(3):
+        buf.zero_()
+        torch.cuda.synchronize()
+        K.convert_rows(w16, w)
+        K.gemm_generic(x, w, out)
+        assert torch.equal(out, want)
+
+
 def test_float32_products_of_more_tokens_than_one_call_makes_ready(K):
     """The tokens' parts take scratch memory, which is filled and used several times over for long prompts."""
     K_, N = 14336, 130

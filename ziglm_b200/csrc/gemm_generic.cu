@@ -146,6 +146,7 @@ struct SegArgs {
     long ldx, ldw, ldy;
     int seg, segs;           // length and number of the segments
     int parts;               // blocks of a cluster; each owns segs / parts neighbouring segments
+    int bound;               // W is older than every kernel that may still run: it is read before the kernel before has ended
 };
 
 __device__ int split_error;                 // first bounded wait that ran out (tc::ERR_*)
@@ -422,6 +423,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SegArgs a) {
             ahead += G;
         };
         if constexpr (!WIDE) {
+            if (!a.bound) pdl_wait();
 #pragma unroll 1
             for (int s = 0; s < OWN - 1; ++s) fetch();
         }
@@ -475,8 +477,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SegArgs a) {
         cp_async_wait<0>();                                                  // gives up with no copy in flight
     } else if (warp == C::LOAD) {
         // ------------------------------------------------------------ weights as they lie in memory
-        // they do not depend on the kernel before: the first are asked for before it has ended
+        // bound weights do not depend on the kernel before: the first are asked for before it has ended
         if (WIDE && lane == 0) {
+            if (!a.bound) pdl_wait();
             int st = 0;
             for (; st < n_stages; ++st) {
                 const int slot = st % C::STAGES_W;
@@ -807,11 +810,12 @@ static int split_chunk(int M, int K) {
 }
 
 static int launch_float(const void* X, const void* W, const void* bias, int bias_dtype, void* Y, int accumulate, int M, int N,
-                        int K, long ldx, long ldw, long ldy, void* scratch, long scratch_bytes, cudaStream_t stream) {
+                        int K, long ldx, long ldw, long ldy, int bound, void* scratch, long scratch_bytes, cudaStream_t stream) {
     if (bias != nullptr && bias_dtype != ZLM_F32 && bias_dtype != ZLM_BF16) return ZLM_ERR_UNSUPPORTED;
     SegArgs a;
     a.X = (const float*)X; a.W = (const float*)W; a.bias = bias; a.Y = (float*)Y;
     a.planes = nullptr;
+    a.bound = bound;
     a.bias_dtype = bias_dtype; a.accumulate = accumulate;
     a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldy = ldy;
     a.segs = segment_count(K);
@@ -884,7 +888,7 @@ ZLM_EXPORT int zlm_gemm_generic(const void* X, int x_dtype, const void* W, int w
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || ldx < K || ldw < K || ldy < N) return ZLM_ERR_BAD_ARG;
     if (x_dtype == ZLM_F32 && w_dtype == ZLM_F32 && y_dtype == ZLM_F32)
-        return launch_float(X, W, bias, bias_dtype, Y, accumulate, M, N, K, ldx, ldw, ldy, nullptr, 0, stream);
+        return launch_float(X, W, bias, bias_dtype, Y, accumulate, M, N, K, ldx, ldw, ldy, 0, nullptr, 0, stream);
     if (x_dtype == ZLM_F32 && w_dtype == ZLM_F32)
         return y_dtype == ZLM_BF16 ? pick_bias<float, float, __nv_bfloat16>(bias_dtype, X, W, bias, Y, accumulate, M, N, K, ldx,
                                                                             ldw, ldy, stream)
@@ -902,15 +906,17 @@ ZLM_EXPORT int zlm_gemm_generic(const void* X, int x_dtype, const void* W, int w
 }
 
 // The same product of float operands, which is faster with scratch memory from 65 tokens on (16-byte aligned; its
-// contents are of no use afterwards).  zlm_gemm_float_scratch: the bytes it takes.
+// contents are of no use afterwards).  zlm_gemm_float_scratch: the bytes it takes.  bound != 0: W holds what it is to hold
+// before any kernel that may still run when this one starts (a model's weights); its first rows are then read while the
+// kernels before finish.  Otherwise W may come from the kernel just before.
 ZLM_EXPORT long zlm_gemm_float_scratch(int M, int K) { return M <= 64 || K <= 0 ? 0 : split_chunk(M, K) * split_row_bytes(K); }
 
 ZLM_EXPORT int zlm_gemm_float(const void* X, const void* W, const void* bias, int bias_dtype, void* Y, int accumulate, int M,
-                              int N, int K, long ldx, long ldw, long ldy, void* scratch, long scratch_bytes,
+                              int N, int K, long ldx, long ldw, long ldy, int bound, void* scratch, long scratch_bytes,
                               cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || ldx < K || ldw < K || ldy < N) return ZLM_ERR_BAD_ARG;
-    return launch_float(X, W, bias, bias_dtype, Y, accumulate, M, N, K, ldx, ldw, ldy, scratch, scratch_bytes, stream);
+    return launch_float(X, W, bias, bias_dtype, Y, accumulate, M, N, K, ldx, ldw, ldy, bound, scratch, scratch_bytes, stream);
 }
 
 // Reads and clears the error word the float kernels report bounded-wait failures through (synchronises the device).

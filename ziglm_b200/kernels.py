@@ -140,7 +140,7 @@ _PROTOTYPES = {
         "zlm_gemm_generic": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
                              c_int, c_long, c_long, c_long, c_void_p],
         "zlm_gemm_float": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_long, c_long, c_long,
-                           c_void_p, c_long, c_void_p],
+                           c_int, c_void_p, c_long, c_void_p],
         "zlm_gemm_float_scratch": [c_int, c_int],
         "zlm_gemm_generic_status": [c_void_p],
     },
@@ -1115,10 +1115,11 @@ def fill_normal(out: torch.Tensor, key: int, mean: float, std: float) -> None:
 
 # ------------------------------------------------------------------------ gemm
 def gemm_generic(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
-                 accumulate: bool = False) -> None:
+                 accumulate: bool = False, weights_bound: bool = False) -> None:
     """out[M,N] (+)= x[M,K] @ w[N,K]^T (+ bias) for any types and sizes; rows may be strided.  Float operands and a float
     result: on the tensor cores in three bf16 parts an operand, with a smaller error than one fmaf a product; else on the
-    CUDA cores."""
+    CUDA cores.  ``weights_bound``: ``w`` holds a model's weights, which no kernel that may still run writes; the float
+    product then reads them while the kernels before it finish.  Without it ``w`` may come from the kernel just before."""
     for t, n in ((x, "x"), (w, "w"), (out, "out")):
         if not t.is_cuda:
             raise KernelError(f"{n} must be on a CUDA device (there is no CPU path)")
@@ -1142,7 +1143,7 @@ def gemm_generic(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Opti
         _check(_fn("gemm_generic", "zlm_gemm_float")(
             x.data_ptr(), w.data_ptr(), _ptr(bias), code(bias.dtype) if bias is not None else F32, out.data_ptr(),
             int(accumulate), M, N, K, x.stride(0) if M > 1 else K, w.stride(0) if N > 1 else K,
-            out.stride(0) if M > 1 else N, _ptr(scratch), size, _stream()), "gemm_float")
+            out.stride(0) if M > 1 else N, int(weights_bound), _ptr(scratch), size, _stream()), "gemm_float")
         return
     _check(_fn("gemm_generic", "zlm_gemm_generic")(
         x.data_ptr(), code(x.dtype), w.data_ptr(), code(w.dtype), _ptr(bias),

@@ -48,7 +48,7 @@ class Linear:
             raise ValueError(f"linear: input width {x.shape[-1]} does not match the weight's {self.in_features}")
         if kernels.fast_gemm(self, x, out, accumulate):
             return out
-        kernels.gemm_generic(x, self.weight, out, bias=self.bias, accumulate=accumulate)
+        kernels.gemm_generic(x, self.weight, out, bias=self.bias, accumulate=accumulate, weights_bound=True)
         return out
 
     def with_activation(self, x: torch.Tensor, out: torch.Tensor, activation: str) -> bool:
@@ -71,6 +71,6 @@ class Linear:
         ssq = step.ws.buf(name + "_ssq", (T, -(-d // 128)), torch.float32)
         done = kernels.fast_gemm(self, x, residual, True, norm_out=(norm.weight, norm.weight_offset, hb, ssq))
         if not done:
-            kernels.gemm_generic(x, self.weight, residual, bias=self.bias, accumulate=True)
+            kernels.gemm_generic(x, self.weight, residual, bias=self.bias, accumulate=True, weights_bound=True)
             return None
         return NormedInput(hb, ssq, norm.eps) if done == 2 else None
