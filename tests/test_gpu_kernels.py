@@ -233,6 +233,63 @@ def test_float32_products_at_the_ends_of_the_range(K, M):
     assert torch.equal(out, x[:, :N])
 
 
+@pytest.mark.parametrize("M", [1, 17, 64, 200])
+@pytest.mark.parametrize("N,K_", [(130, 523), (200, 8200)])
+def test_float32_products_with_many_results_that_are_not_finite(K, M, N, K_):
+    """Whole rows and columns of results that are NaN or infinite: what float gives, the other results untouched, and no
+    wait of the kernel runs out meanwhile."""
+    inf, nan = float("inf"), float("nan")
+    x, w = rnd((M, K_), torch.float32, seed=61).to(DEV), rnd((N, K_), torch.float32, seed=62).to(DEV)
+    plain = torch.empty(M, N, device=DEV)
+    K.gemm_generic(x, w, plain)
+    far = K_ - 3
+    for name, xs, ws in (("all tokens NaN", torch.full_like(x, nan), w), ("a NaN in every token", x.index_fill(1, torch.tensor([far], device=DEV), nan), w),
+                         ("an infinity in every token", x.index_fill(1, torch.tensor([far], device=DEV), inf), w),
+                         ("tokens of infinities", x.abs() + inf, w.abs()), ("one token", x.index_fill(0, torch.tensor([M // 2], device=DEV), -inf), w),
+                         ("one row of weights", x, w.index_fill(0, torch.tensor([77], device=DEV), inf)),
+                         ("an infinity in nine rows", x, torch.cat([w[:20], w[20:29].index_fill(1, torch.tensor([1], device=DEV), inf), w[29:]])),
+                         ("a large number in every row", x.index_fill(1, torch.tensor([5], device=DEV), 0.25),
+                          w.index_fill(1, torch.tensor([5], device=DEV), torch.finfo(torch.float32).max))):
+        out = torch.empty(M, N, device=DEV)
+        K.gemm_generic(xs, ws, out)
+        want = xs.double() @ ws.double().t()
+        assert torch.equal(out.isnan(), want.isnan()), name
+        assert torch.equal(out == inf, want == inf) and torch.equal(out == -inf, want == -inf), name
+        same = (xs == x).all(1)[:, None] & (ws == w).all(1)[None, :]
+        assert torch.equal(out[same], plain[same]), name
+        if "large" in name:
+            bound = 16 * 2.0 ** -24 * (xs.double().abs() @ ws.double().abs().t())
+            assert ((out.double() - want).abs() <= bound).all()
+    assert K.gemm_generic_status() == 0
+
+
+def test_float32_products_that_are_not_finite_take_their_time_in_bounds(K):
+    """One row of weights that is not finite: every token's result in that row is summed again."""
+    M, N, K_ = 64, 2048, 8192
+    x, w = rnd((M, K_), torch.float32, seed=63).to(DEV), rnd((N, K_), torch.float32, seed=64).to(DEV)
+    bad = w.clone()
+    bad[300] = float("inf")
+    out = torch.empty(M, N, device=DEV)
+
+    def us(weights, tokens):
+        times = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            K.gemm_generic(tokens, weights, out)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b) * 1e3)
+        return sorted(times)[2]
+
+    finite = us(w, x)
+    row, tokens, every = us(bad, x.abs()), us(w, x.index_fill(1, torch.tensor([9], device=DEV), float("inf"))), us(w, x * float("nan"))
+    print(f"finite {finite:.0f} us, a row {row:.0f}, every token {tokens:.0f}, all NaN {every:.0f}")
+    # a row: 32 results a warp of 32 coalesced reads each; one thread's 32,768 dependent ones took tens of milliseconds
+    assert row < 20 * finite and every < 20 * finite and tokens < 100 * finite
+    assert K.gemm_generic_status() == 0
+
+
 @pytest.mark.parametrize("wide", [True, False])
 @pytest.mark.parametrize("M", [1, 40, 200])
 def test_float32_products_with_weights_from_the_kernel_before(K, wide, M):

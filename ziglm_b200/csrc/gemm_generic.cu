@@ -118,8 +118,8 @@ gemm_generic_kernel(const TX* __restrict__ X, const TW* __restrict__ W, const TB
 // The order of an output's additions is fixed by K alone (the segments above, the periods, one order of the products
 // in a period): a value does not depend on M, on where the row sits in the batch or on the tile it falls in.
 //
-// A result that is not finite is summed again with fmaf: a part of an infinity, or of a number that bf16 rounds up to
-// one, makes NaN where float has an answer.
+// A result that is not finite is summed again with fmaf (sum_again): a part of an infinity, or of a number that bf16 rounds
+// up to one, makes NaN where float has an answer.
 //
 // Error against 64 bits, relative, of sums of normal numbers: 1.0e-7 over K = 4096 and 1.3e-7 over K = 14336 (one fmaf a
 // product in at most eight segments: 5.7e-7, 7.6e-7).  With 32, 128 or 1024 k a period 1.2e-7, 1.4e-7, 9.9e-7: shorter
@@ -345,6 +345,44 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* X, long ld
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+// A warp's results of a segment (`sums`: this lane's weight row, `tokens` of them), those that are not finite summed again over
+// n k of the tokens' rows `x` and this lane's row `w` (null: there is none), by the whole warp: the first eight k a row a lane,
+// which is all where the token's numbers are NaN; then row after row, the lanes on neighbouring k.  A sum that is NaN stays
+// so, and is left there.  No wait of the kernel runs out meanwhile: a poll takes 4 us, the limit is 17 s.
+// 64 x 2048 x 8192, of which are not finite: one row of weights 90 us, one number of every token 2,440, all tokens' numbers
+// 140 (finite 58; a thread by itself with 32 sums one after another took tens of milliseconds for the first).
+// A function of its own, called with everything in memory: inlined it cost the way past it registers and 2 percent.
+__device__ __noinline__ void sum_again(float* sums, int tokens, const float* x, long ldx, const float* w, int n, int lane) {
+#pragma unroll 1
+    for (int t = 0; t < tokens; ++t, x += ldx) {
+        unsigned who = __ballot_sync(0xffffffffu, w != nullptr && !(fabsf(sums[t]) <= 3.402823466e38f));
+        if (who == 0) continue;
+        float v = 0.f;
+        const bool mine = (who >> lane) & 1u;
+        if (mine)
+            for (int k = 0; k < min(n, 8); ++k) v = fmaf(x[k], w[k], v);
+        for (who &= __ballot_sync(0xffffffffu, v == v); who != 0; who &= who - 1) {
+            const int l = __ffs(who) - 1;
+            const float* row = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, (unsigned long long)w, l));
+            float sum = 0.f;
+            for (int k = lane; k - lane < n && !__any_sync(0xffffffffu, sum != sum); k += 256) {
+                float p[8], q[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const bool have = k + 32 * i < n;
+                    p[i] = have ? x[k + 32 * i] : 0.f;
+                    q[i] = have ? row[k + 32 * i] : 0.f;
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) sum = fmaf(p[i], q[i], sum);
+            }
+            sum = warp_sum(sum);
+            if (lane == l) v = sum;
+        }
+        if (mine) sums[t] = v;
+    }
 }
 
 // Roles of the warps.  One thread asks for the weights (TMA, 128 rows x 32 k a stage); with rows off 16-byte boundaries
@@ -652,24 +690,19 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SegArgs a) {
                 tc::tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(seg_free);
-                unsigned long long again = 0;                                // results that are not finite
+                bool again = false;                                          // results that are not finite
 #pragma unroll
-                for (int i = 0; i < COLS; ++i)
-                    if (!(fabsf(acc[i]) <= 3.402823466e38f)) again |= 1ull << i;
-                while (again != 0) {
-                    const int t = __ffsll((long long)again) - 1;
-                    again &= again - 1;
-                    if (gn >= a.N || m0 + t0 + t >= a.M) continue;
-                    const int n = min(a.seg, k_hi - k_lo - s * a.seg);
-                    const float* x = a.X + (long)(m0 + t0 + t) * a.ldx + k_lo + s * a.seg;
-                    const float* w = a.W + (long)gn * a.ldw + k_lo + s * a.seg;
-                    float v = 0.f;
-#pragma unroll 1
-                    for (int k = 0; k < n; ++k) v = fmaf(x[k], w[k], v);
+                for (int i = 0; i < COLS; ++i) again |= !(fabsf(acc[i]) <= 3.402823466e38f);
+                if (__builtin_expect(__any_sync(0xffffffffu, again && gn < a.N), 0)) {
+                    float all[COLS];
 #pragma unroll
-                    for (int i = 0; i < COLS; ++i) acc[i] = i == t ? v : acc[i];
+                    for (int i = 0; i < COLS; ++i) all[i] = acc[i];
+                    const int k0 = k_lo + s * a.seg;
+                    sum_again(all, min(COLS, a.M - m0 - t0), a.X + (long)(m0 + t0) * a.ldx + k0, a.ldx,
+                              gn < a.N ? a.W + (long)gn * a.ldw + k0 : nullptr, min(a.seg, k_hi - k0), lane);
+#pragma unroll
+                    for (int i = 0; i < COLS; ++i) acc[i] = all[i];
                 }
-                __syncwarp();
             }
             // neighbouring segments are added pairwise, then the pairs, then the fours: the sums that wait for their
             // other half lie in tensor memory, a level each (128 tokens: in shared memory, one level)
