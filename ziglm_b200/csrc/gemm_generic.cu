@@ -109,8 +109,10 @@ gemm_generic_kernel(const TX* __restrict__ X, const TW* __restrict__ W, const TB
 // ------------------------------------------------- float operands: tensor cores, every operand in three bf16 parts
 // A float is the sum of three bf16 numbers, a = a0 + a1 2^-8 + a2 2^-16, each the rounded rest of what came before it
 // (the factors keep the parts in the range of a itself, so that no part of a normal number is lost among the smallest
-// bf16 numbers).  Of the nine products of parts the six largest are taken, on the tensor cores with 32-bit sums:
-// what is left out is below 2^-25 of a product, half a rounding of one fmaf.  They go to three sums in tensor memory,
+// bf16 numbers); the idea is published (Henry, Tang, Heinecke: Leveraging the bfloat16 artificial intelligence datatype for
+// higher-precision computations, 2019).  Of the nine products of parts the six largest are taken, on the tensor cores with
+// 32-bit sums: what is left out is at most 2^-24 of a product, a rounding of one fmaf (a = b = 1 + 2^-8 - 2^-17), and
+// mostly a tenth of that.  They go to three sums in tensor memory,
 // g0 = a0 b0, g1 = a0 b1 + a1 b0, g2 = a0 b2 + a1 b1 + a2 b0.  The tensor core cuts what does not fit a 32-bit sum
 // instead of rounding it, so g0 holds SPLIT_PERIOD k at a time and threads add it up in registers, rounded; g1 and g2
 // are added 2^8 and 2^16 times smaller at the end of a segment, where the cuts do not count.
@@ -125,12 +127,17 @@ gemm_generic_kernel(const TX* __restrict__ X, const TW* __restrict__ W, const TB
 // product in at most eight segments: 5.7e-7, 7.6e-7).  With 32, 128 or 1024 k a period 1.2e-7, 1.4e-7, 9.9e-7: shorter
 // periods round oftener, longer ones cut oftener (a bias of -4.9e-8 with 64).
 //
-// Measured against FFMA tiles and streaming kernels: 600 tokens x 28672 x 4096 3357 -> 927 us, 600 x 4096 x 14336
-// 1816 -> 411, 64 x 28672 x 4096 393 -> 179, 20 x 28672 x 4096 243 -> 121, 8 x 28672 x 4096 117 -> 111 (4.6 TB/s),
-// 1 x 2048 x 8192 24 -> 31.  Up to 64 tokens the weights' bytes and a block's start and end (some 8 us) bound it; with
-// 128 tokens a stage takes about 1,250 cycles of which the instructions are 768: splitting and adding up share the issue
-// slots (without the splitting 858 us of 943, without the small products 836, without both 706).  Two blocks as one
-// (cta_group::2, 256 x 128) took 1370 us: its hand-overs between the SMs are longer than what it saves in loads.
+// Measured in a captured run of launches against FFMA tiles and streaming kernels: 600 tokens x 28672 x 4096 3351 -> 943 to
+// 989 us, 600 x 4096 x 14336 1809 -> 412, 64 x 28672 x 4096 387 -> 147, 32 x 28672 x 4096 224 -> 99, 8 x 28672 x 4096 99 -> 79
+// (6.0 TB/s).  Fewer than 8 tokens on few weight rows or a short K lose: 1 x 2048 x 8192 15 -> 22, 1 x 5120 x 5120 22 -> 29,
+// 1 x 5120 x 13824 56 -> 63 to 72, 1 x 4096 x 4096 15.0 -> 16.9, 1 x 1024 x 256 2.7 -> 4.6, and one of at most 65 to 128 tokens
+// with K = 64 7.1 -> 8.9; all of float32 decoding gains or stays (1 sequence at the 1B and 8B shapes 605 -> 579, 1,201 ->
+// 1,209 us, four layers) but for one or two sequences at the 13B shape (1,255 -> 1,325).  A launch's start and end take some 7 us
+// there and a block's stage, one block an SM, some 450 ns: its waits and hand-overs, not its bytes.  Without effect on that or
+// slower, each with the same bits: a second sum for g0, three buffers of weights, a second issuing warp, a0's products in one
+// instruction of 48 columns, tokens split ahead of their buffer by two groups of warps.  With 128 tokens splitting and adding
+// up share the issue slots (without the splitting 858 us of 943, without the small products 836, without both 706).  Two
+// blocks as one (cta_group::2, 256 x 128) took 1370 us: its hand-overs between the SMs are longer than what it saves in loads.
 constexpr int SPLIT_K = 32;                 // k of a stage: 128 bytes of float, two tensor-core instructions' worth
 constexpr int SPLIT_ROWS = 128;             // weight rows of a tile: the instruction's M, a lane of tensor memory each
 constexpr int SPLIT_PERIOD = 64;            // k whose products meet in the tensor core before a rounded addition
@@ -292,10 +299,12 @@ __device__ __forceinline__ void add_parts(const SegArgs& a, uint32_t part, int r
     }
 }
 
-// One warp's rows of a stage, R rows from `src` on (row r of them at most `last`, which is repeated), k0..k0+31 of a
-// row in 128 bytes of shared memory, 16-byte piece c of row r at piece c ^ (r & 7).  k from k_end on are zeros.
+// One warp's rows of a stage, the first `rows` of R rows from `src` on, k0..k0+31 of a row in 128 bytes of shared memory,
+// 16-byte piece c of row r at piece c ^ (r & 7).  Rows from `rows` on and k from k_end on are zeros and not read (`src`
+// is a row that exists): rows that repeated the last one asked a single token's lines 16 times over in
+// every block (1 x 28672 x 4096 93 -> 82 us).
 template <int R, bool WIDE>
-__device__ __forceinline__ void copy_rows(uint32_t dst, const float* src, long ld, int last, int k0, int k_end, int lane) {
+__device__ __forceinline__ void copy_rows(uint32_t dst, const float* src, long ld, int rows, int k0, int k_end, int lane) {
     if constexpr (WIDE) {
         const int c = lane & 7, k = k0 + 4 * c;
         const bool have = k < k_end;                        // K is a multiple of 4: a piece is whole or absent
@@ -303,14 +312,15 @@ __device__ __forceinline__ void copy_rows(uint32_t dst, const float* src, long l
 #pragma unroll
         for (int i = 0; i < (R + 3) / 4; ++i) {
             const int r = 4 * i + (lane >> 3);
-            cp_async_16(dst + r * 128 + ((c ^ (r & 7)) << 4), from + (long)min(r, last) * ld, have ? 16 : 0);
+            cp_async_16(dst + r * 128 + ((c ^ (r & 7)) << 4), r < rows ? from + (long)r * ld : from, have && r < rows ? 16 : 0);
         }
     } else {
         const bool have = k0 + lane < k_end;
         const float* from = src + (have ? k0 + lane : 0);
 #pragma unroll 4
         for (int r = 0; r < R; ++r)
-            cp_async_4(dst + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4, from + (long)min(r, last) * ld, have ? 4 : 0);
+            cp_async_4(dst + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4, r < rows ? from + (long)r * ld : from,
+                       have && r < rows ? 4 : 0);
     }
 }
 
@@ -397,10 +407,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SegArgs a) {
     extern __shared__ uint8_t split_smem[];
     const uint32_t raw = tc::smem_u32(split_smem), base = (raw + 1023u) & ~1023u;
     const uint32_t ring_x = base + C::STAGES_W * C::RAW_W, planes = base + C::RINGS, kept = planes + C::BUFS * C::PLANES, bars = kept + C::KEPT;
-    // barriers: weights' parts ready [2] and read [2], tokens ready [BUFS] and read [BUFS], the sums of a period and of a
-    // segment ready and read, no instruction in flight, weights in memory ready [STAGES_W] and read [STAGES_W]; then the
+    // barriers: weights' parts ready [2] and read [2] (tokens that are split here share them: one wait and one commit a stage
+    // less, 6144 x 4096 at 8 tokens 25.4 -> 24.2 us, at 64 44.8 -> 41.5), planes ready [BUFS] and read [BUFS], the sums of a
+    // period and of a segment ready and read, no instruction in flight, weights in memory ready [STAGES_W] and read [STAGES_W]; then the
     // tensor memory's address and the abort flag
-    const uint32_t w_full = bars, w_empty = bars + 16, x_full = bars + 32, x_empty = bars + 64;
+    const uint32_t w_full = bars, w_empty = bars + 16;
+    const uint32_t x_full = C::PRE ? bars + 32 : w_full, x_empty = C::PRE ? bars + 64 : w_empty;   // one pair for both
     const uint32_t sums_full = bars + 96, sums_free = bars + 104, seg_full = bars + 112, seg_free = bars + 120, drained = bars + 128;
     const uint32_t raw_full = bars + 136, raw_empty = raw_full + 8 * C::STAGES_W;
     uint32_t* holder = reinterpret_cast<uint32_t*>(split_smem + (bars - raw) + 136 + 16 * C::STAGES_W);
@@ -417,11 +429,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SegArgs a) {
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; ++s) {
-            tc::mbar_init(w_full + 8 * s, 4);
+            tc::mbar_init(w_full + 8 * s, C::PRE ? 4 : 8);
             tc::mbar_init(w_empty + 8 * s, 1);
         }
-        for (int s = 0; s < C::BUFS; ++s) {
-            tc::mbar_init(x_full + 8 * s, C::PRE ? 1 : 4);
+        for (int s = 0; C::PRE && s < C::BUFS; ++s) {
+            tc::mbar_init(x_full + 8 * s, 1);
             tc::mbar_init(x_empty + 8 * s, 1);
         }
         for (int s = 0; s < C::STAGES_W; ++s) {
@@ -450,13 +462,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SegArgs a) {
         // ------------------------------------------------------------ weights into their parts
         constexpr int G = C::GROUPS, OWN = C::STAGES_W / G;                  // slots of the ring a group fills itself
         const int w = warp & 3, group = warp >> 2;
-        const int first = min(n0 + 32 * w, a.N - 1), last = a.N - 1 - first;
-        const float* src = a.W + (long)first * a.ldw;
+        const int rows = a.N - (n0 + 32 * w);
+        const float* src = a.W + (long)min(n0 + 32 * w, a.N - 1) * a.ldw;
         const uint32_t mine = base + 32 * w * 128;
         int ahead = group;
         auto fetch = [&]() {
             const int slot = group * OWN + ahead / G % OWN;
-            if (ahead < n_stages) copy_rows<32, false>(mine + slot * C::RAW_W, src, a.ldw, last, k_lo + ahead * SPLIT_K, k_hi, lane);
+            if (ahead < n_stages) copy_rows<32, false>(mine + slot * C::RAW_W, src, a.ldw, rows, k_lo + ahead * SPLIT_K, k_hi, lane);
             cp_async_commit();
             ahead += G;
         };
@@ -549,11 +561,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SegArgs a) {
         // ------------------------------------------------------------ tokens into their parts
         constexpr int XR = TOK / 4;                                          // a warp's token rows
         const int w = warp & 3;
-        const int first = min(m0 + XR * w, a.M - 1), last = a.M - 1 - first;
-        const float* src = a.X + (long)first * a.ldx;
+        const int rows = a.M - (m0 + XR * w);
+        const float* src = a.X + (long)min(m0 + XR * w, a.M - 1) * a.ldx;
         const uint32_t ring = ring_x + XR * w * 128;
         auto fetch = [&](int st) {
-            if (st < n_stages) copy_rows<XR, WIDE>(ring + (st % C::STAGES_X) * C::RAW_X, src, a.ldx, last, k_lo + st * SPLIT_K, k_hi, lane);
+            if (st < n_stages) copy_rows<XR, WIDE>(ring + (st % C::STAGES_X) * C::RAW_X, src, a.ldx, rows, k_lo + st * SPLIT_K, k_hi, lane);
             cp_async_commit();
         };
         pdl_wait();
@@ -601,27 +613,25 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SegArgs a) {
         // ------------------------------------------------------------ tensor-core instructions
         constexpr uint32_t one = tc::idesc_bf16(128, TOK), two = tc::idesc_bf16(128, 2 * TOK);
         int in_seg = 0, period = 0, segment = 0, st = 0;
+        // a segment is an even number of stages and starts a period: a stage's buffer and its place in the period go together
+        static_assert(PERIOD == 2 && C::BUFS % 2 == 0, "two stages a period, two buffers of weights");
+        // (two stages at a time spill at 16 and 32 tokens: 1 x 2048 x 8192 23.7 us, 22.4 without; at 128 they save 3 percent)
+#pragma unroll (TOK <= 32 ? 1 : 2)
         for (; st < n_stages; ++st) {
-            const int buf = st & 1, xb = st % C::BUFS;
-            const bool starts = in_seg % PERIOD == 0, seg_ends = in_seg + 1 == seg_stages || st + 1 == n_stages;
-            const bool ends = (in_seg + 1) % PERIOD == 0 || seg_ends;
-            if (!tc::warp_wait(x_full + 8 * xb, (st / C::BUFS) & 1, abort_flag, err, tc::ERR_WAIT_FULL)) break;
+            const int buf = st & 1, xb = C::PRE ? st % C::BUFS : buf;
+            const bool starts = buf == 0, seg_ends = in_seg + 1 == seg_stages || st + 1 == n_stages, ends = buf == 1 || seg_ends;
+            if (C::PRE && !tc::warp_wait(x_full + 8 * xb, (st / C::BUFS) & 1, abort_flag, err, tc::ERR_WAIT_FULL)) break;
             if (!tc::warp_wait(w_full + 8 * buf, (st >> 1) & 1, abort_flag, err, tc::ERR_WAIT_FULL)) break;
             if (starts && period > 0 && !tc::warp_wait(sums_free, (period - 1) & 1, abort_flag, err, tc::ERR_WAIT_ACCUM)) break;
             tc::tc_fence_after_sync();
             const uint32_t A = tmem + C::A0 + 48 * buf;
             const uint64_t B0 = smem_desc_sw64(planes + xb * C::PLANES), B1 = smem_desc_sw64(planes + xb * C::PLANES + C::PLANE);
-            if (tc::elect_one()) {
+            auto large = [&]() {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) tc::umma_bf16_ts(tmem, A + 8 * h, B0 + 2 * h, one, !(starts && h == 0));
                 if (ends) tc::umma_commit(sums_full);                        // g0 is read while g1 and g2 are summed
-            }
-            __syncwarp();
-            if (in_seg == 0 && segment > 0) {
-                if (!tc::warp_wait(seg_free, (segment - 1) & 1, abort_flag, err, tc::ERR_WAIT_ACCUM)) break;
-                tc::tc_fence_after_sync();
-            }
-            if (tc::elect_one()) {
+            };
+            auto small = [&]() {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     tc::umma_bf16_ts(tmem + TOK, A + 8 * h, B1 + 2 * h, two, !(in_seg == 0 && h == 0));
@@ -629,8 +639,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, SegArgs a) {
                     tc::umma_bf16_ts(tmem + 2 * TOK, A + 32 + 8 * h, B0 + 2 * h, one, 1);
                 }
                 tc::umma_commit(w_empty + 8 * buf);
-                tc::umma_commit(x_empty + 8 * xb);
+                if (C::PRE) tc::umma_commit(x_empty + 8 * xb);
                 if (seg_ends) tc::umma_commit(seg_full);
+            };
+            if (in_seg == 0 && segment > 0) {
+                if (tc::elect_one()) large();
+                __syncwarp();
+                if (!tc::warp_wait(seg_free, (segment - 1) & 1, abort_flag, err, tc::ERR_WAIT_ACCUM)) break;
+                tc::tc_fence_after_sync();
+                if (tc::elect_one()) small();
+            } else if (tc::elect_one()) {
+                large();
+                small();
             }
             __syncwarp();
             if (ends) ++period;
