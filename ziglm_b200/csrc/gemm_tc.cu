@@ -86,7 +86,7 @@ struct TcArgs {
 __host__ __device__ constexpr int sub_rows(int bn) { return (bn == 16 || bn == 64) ? 16 : 32; }
 
 // DEEP: 0 the usual number of stages, n > 0 n stages; SPLIT_K + n: n stages and no staging area, for launches that
-// split K (their sums meet in the stages' memory).
+// split K (their sums meet in the stages' memory, with tiles of 32 and 64 tokens in memory of their own).
 constexpr int SPLIT_K = 100;
 
 template <int BN, int DEEP = 0> struct TcCfg {
@@ -95,10 +95,10 @@ template <int BN, int DEEP = 0> struct TcCfg {
     // DEEP: the gated product of a decode step, and any whole product of more tiles than SMs, runs as one tile of a
     // megabyte of weights per block, at most two blocks per SM; what bounds it is the bytes each block has in flight, so
     // it takes a fourth stage (measured: five and more cost the next product its early residence).
-    // A product whose K is split takes four stages in the same room (no staging area), and five or six where there is at
-    // most one block an SM and more K blocks than four: a small product's weights (four K blocks a block) are then all
-    // requested before the kernel before it ends, and a lone block has enough bytes in flight for its SM's share of
-    // the memory's bandwidth.
+    // A product whose K is split takes four stages in the same room (no staging area; three with tiles of 64 tokens, beside
+    // the memory the sums arrive in), and with tiles of 16 tokens six where there is at most one block an SM and more K
+    // blocks than four: a small product's weights (four K blocks a block) are then all requested before the kernel before
+    // it ends, and a lone block has enough bytes in flight for its SM's share of the memory's bandwidth.
     static constexpr bool SPLIT = DEEP >= SPLIT_K;
     static constexpr int STAGES = SPLIT ? DEEP - SPLIT_K : BN <= 32 ? (DEEP ? DEEP : 3) : (BN == 128 ? 5 : 4);
     static constexpr int B_BYTES = BN * TC_BK * 2;
@@ -247,7 +247,7 @@ __device__ __forceinline__ void store_tile(const TcArgs& a, const CUtensorMap* t
 // leave: a step of 64 sequences at the 1B shape 1262 -> 1185 us, of 24 909 -> 858.  Narrower tiles keep that form: a third
 // block would not fit an SM beside memory for the sums, and pushing them into the stages once all ranks are done, behind one
 // more barrier, took 693 us for one sequence against 681.)
-template <class C, int BN, int MODE>
+template <int BN, int MODE>
 __device__ __forceinline__ void push_and_store(const TcArgs& a, uint32_t rank, uint32_t tmem_base, uint32_t recv_addr,
                                                const uint8_t* recv_at, const float* inv_s, uint32_t acc_full,
                                                int n_kb, volatile int* abort_flag) {
@@ -416,11 +416,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     float* partial = reinterpret_cast<float*>(smem);   // split-K only (one tile per block): [BN][128] floats
 
     __shared__ float inv_s[64];                     // row scales of a product that completes a norm
-    __shared__ float norm_red[2][4][4];             // sums of squares: [epilogue half][token of a group][warp]
+    __shared__ float norm_red[2][4];                // sums of squares: [epilogue half][warp]
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-    constexpr bool MAY_SPLIT = C::SPLIT || BN > 64;  // narrow tiles have a form of their own for split launches
-    const bool split = MAY_SPLIT && a.splits > 1;
-    const uint32_t rank = split ? cluster_rank() : 0u;
+    const uint32_t rank = C::SPLIT ? cluster_rank() : 0u;   // split launches (tiles of at most 64 tokens) are forms of their own
     const int kb0 = (int)rank * a.kb_per_split;
     int n_kb = a.kb_total - kb0;
     if (n_kb > a.kb_per_split) n_kb = a.kb_per_split;
@@ -559,9 +557,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
         const uint32_t part_addr = smem_u32(partial);
         int local = 0;
         if constexpr (C::PUSH) {
-            push_and_store<C, BN, MODE>(a, rank, tmem_base, stage_out, smem + (stage_out - base), inv_s, acc_full0, n_kb, abort_flag);
+            push_and_store<BN, MODE>(a, rank, tmem_base, stage_out, smem + (stage_out - base), inv_s, acc_full0, n_kb, abort_flag);
             first_cluster_barrier_done = true;
-        } else if (split) {
+        } else if constexpr (C::SPLIT) {
             // ---- K is split over the cluster: one tile per block.  Every rank parks its partial
             // accumulator in its own shared memory; then rank r sums, in rank order, a slice of the
             // tile's token columns over all ranks and writes that slice.
@@ -609,131 +607,56 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             uint32_t remote[8];
 #pragma unroll
             for (int r = 0; r < 8; ++r) remote[r] = r < a.splits ? map_to_rank(part_addr, (uint32_t)r) : 0u;
-            // Up to EB tokens of this warp at a time (tiles of 64 tokens and more): their partials are all requested before the
-            // first sum, so the latency of the cluster's shared memory is paid once per group, not per token.
-            constexpr int EB = BN >= 64 ? 2 : 1;          // narrow tiles keep their registers: three blocks an SM
-            if constexpr (EB == 1) {
-                for (int cc = c_lo + egroup; cc < c_hi && good; cc += 2) {
-                    const int tok = tok0 + cc;
-                    if (tok >= a.T) break;
-                    float part[8];
-    #pragma unroll
-                    for (int r = 0; r < 8; ++r)
-                        part[r] = r < a.splits ? ld_cluster_f32(remote[r] + 4u * (cc * TC_BM + f_local)) : 0.f;
-                    const float before = ahead;
-                    ahead = residual(cc + 2);
-                    float val = part[0];
-    #pragma unroll
-                    for (int r = 1; r < 8; ++r) val += part[r];
-                    if (a.scale_ssq != nullptr) val *= inv_s[cc];
-                    val += bias_v;
-                    if (!GLU && a.unary_act) val = unary_activation(val, a.unary_act);
-                    if (GLU) {
-                        const float up = __shfl_down_sync(0xffffffffu, val, 1);
-                        const float g = val;
-                        val = gated_pair<MODE == OUT_BF16_GEGLU>(g, up, a.glu_limit, a.glu_slope);
-                    }
-                    if (writer && out_f < out_n) {
-                        if (MODE == OUT_BF16 || GLU)
-                            reinterpret_cast<__nv_bfloat16*>(a.Y)[(long)tok * a.ldy + out_f] = __float2bfloat16_rn(val);
-                        else if (MODE == OUT_F32_ACC && a.norm_gain == nullptr)   // one adder per element: the order is fixed
-                            atomicAdd(reinterpret_cast<float*>(a.Y) + (long)tok * a.ldy + out_f, val);
-                        else if (MODE != OUT_F32_ACC)
-                            reinterpret_cast<float*>(a.Y)[(long)tok * a.ldy + out_f] = val;
-                    }
-                    if (MODE == OUT_F32_ACC && a.norm_gain != nullptr) {
-                        // The only adder of this element sees the finished residual value: it leaves x * gain for
-                        // the product after the norm, and the tile's 128 features of this token give one partial
-                        // sum of squares (four warps of this half of the epilogue, summed in warp order).
-                        float xn = 0.f;
-                        if (out_f < out_n) {
-                            xn = before + val;
-                            reinterpret_cast<float*>(a.Y)[(long)tok * a.ldy + out_f] = xn;
-                            a.norm_hb[(long)tok * a.ld_hb + out_f] = __float2bfloat16_rn(xn * gain);
-                        }
-                        const float sq = warp_sum(xn * xn);
-                        if (lane == 0) norm_red[egroup][0][q] = sq;
-                        if (egroup == 0) asm volatile("bar.sync 3, 128;" ::: "memory");
-                        else asm volatile("bar.sync 4, 128;" ::: "memory");
-                        if (q == 0 && lane == 0)
-                            a.norm_ssq[(long)tok * a.norm_p + tile / tok_tiles] =
-                                ((norm_red[egroup][0][0] + norm_red[egroup][0][1]) + norm_red[egroup][0][2]) + norm_red[egroup][0][3];
-                        if (egroup == 0) asm volatile("bar.sync 3, 128;" ::: "memory");
-                        else asm volatile("bar.sync 4, 128;" ::: "memory");
-                    }
+            for (int cc = c_lo + egroup; cc < c_hi && good; cc += 2) {
+                const int tok = tok0 + cc;
+                if (tok >= a.T) break;
+                float part[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                    part[r] = r < a.splits ? ld_cluster_f32(remote[r] + 4u * (cc * TC_BM + f_local)) : 0.f;
+                const float before = ahead;
+                ahead = residual(cc + 2);
+                float val = part[0];
+#pragma unroll
+                for (int r = 1; r < 8; ++r) val += part[r];
+                if (a.scale_ssq != nullptr) val *= inv_s[cc];
+                val += bias_v;
+                if (!GLU && a.unary_act) val = unary_activation(val, a.unary_act);
+                if (GLU) {
+                    const float up = __shfl_down_sync(0xffffffffu, val, 1);
+                    const float g = val;
+                    val = gated_pair<MODE == OUT_BF16_GEGLU>(g, up, a.glu_limit, a.glu_slope);
                 }
-            } else {
-                for (int cc0 = c_lo + egroup; cc0 < c_hi && good; cc0 += 2 * EB) {
-                    if (tok0 + cc0 >= a.T) break;
-                    bool live[EB];
-                    float val[EB], before[EB];
-    #pragma unroll
-                    for (int u = 0; u < EB; ++u) before[u] = u == 0 ? ahead : residual(cc0 + 2 * u);
-                    ahead = residual(cc0 + 2 * EB);
-                    float part[EB][8];
-    #pragma unroll
-                    for (int u = 0; u < EB; ++u) {
-                        const int cc = cc0 + 2 * u;
-                        live[u] = cc < c_hi && tok0 + cc < a.T;          // the same for every thread of this half
-    #pragma unroll
-                        for (int r = 0; r < 8; ++r)
-                            part[u][r] = (live[u] && r < a.splits) ? ld_cluster_f32(remote[r] + 4u * (cc * TC_BM + f_local)) : 0.f;
+                if (writer && out_f < out_n) {
+                    if (MODE == OUT_BF16 || GLU)
+                        reinterpret_cast<__nv_bfloat16*>(a.Y)[(long)tok * a.ldy + out_f] = __float2bfloat16_rn(val);
+                    else if (MODE == OUT_F32_ACC && a.norm_gain == nullptr)   // one adder per element: the order is fixed
+                        atomicAdd(reinterpret_cast<float*>(a.Y) + (long)tok * a.ldy + out_f, val);
+                    else if (MODE != OUT_F32_ACC)
+                        reinterpret_cast<float*>(a.Y)[(long)tok * a.ldy + out_f] = val;
+                }
+                if (MODE == OUT_F32_ACC && a.norm_gain != nullptr) {
+                    // The only adder of this element sees the finished residual value: it leaves x * gain for
+                    // the product after the norm, and the tile's 128 features of this token give one partial
+                    // sum of squares (four warps of this half of the epilogue, summed in warp order).
+                    float xn = 0.f;
+                    if (out_f < out_n) {
+                        xn = before + val;
+                        reinterpret_cast<float*>(a.Y)[(long)tok * a.ldy + out_f] = xn;
+                        a.norm_hb[(long)tok * a.ld_hb + out_f] = __float2bfloat16_rn(xn * gain);
                     }
-    #pragma unroll
-                    for (int u = 0; u < EB; ++u) {
-                        const int cc = cc0 + 2 * u;
-                        float v = part[u][0];
-    #pragma unroll
-                        for (int r = 1; r < 8; ++r) v += part[u][r];     // in rank order
-                        if (a.scale_ssq != nullptr) v *= inv_s[cc & 63];
-                        v += bias_v;
-                        if (!GLU && a.unary_act) v = unary_activation(v, a.unary_act);
-                        if (GLU) {
-                            const float up = __shfl_down_sync(0xffffffffu, v, 1);
-                            const float g = v;
-                            v = gated_pair<MODE == OUT_BF16_GEGLU>(g, up, a.glu_limit, a.glu_slope);
-                        }
-                        val[u] = v;
-                    }
-    #pragma unroll
-                    for (int u = 0; u < EB; ++u) {
-                        const int tok = tok0 + cc0 + 2 * u;
-                        if (!live[u] || !writer || out_f >= out_n) continue;
-                        if (MODE == OUT_BF16 || GLU)
-                            reinterpret_cast<__nv_bfloat16*>(a.Y)[(long)tok * a.ldy + out_f] = __float2bfloat16_rn(val[u]);
-                        else if (MODE == OUT_F32_ACC && a.norm_gain == nullptr)   // one adder per element: the order is fixed
-                            atomicAdd(reinterpret_cast<float*>(a.Y) + (long)tok * a.ldy + out_f, val[u]);
-                        else if (MODE == OUT_F32_ACC)
-                            reinterpret_cast<float*>(a.Y)[(long)tok * a.ldy + out_f] = before[u] + val[u];
-                        else
-                            reinterpret_cast<float*>(a.Y)[(long)tok * a.ldy + out_f] = val[u];
-                    }
-                    if (MODE == OUT_F32_ACC && a.norm_gain != nullptr) {
-                        // The only adder of an element sees the finished residual value: it leaves x * gain for
-                        // the product after the norm, and the tile's 128 features of a token give one partial
-                        // sum of squares (four warps of this half of the epilogue, summed in warp order).
-    #pragma unroll
-                        for (int u = 0; u < EB; ++u) {
-                            float xn = 0.f;
-                            if (live[u] && out_f < out_n) {
-                                xn = before[u] + val[u];
-                                a.norm_hb[(long)(tok0 + cc0 + 2 * u) * a.ld_hb + out_f] = __float2bfloat16_rn(xn * gain);
-                            }
-                            const float sq = warp_sum(xn * xn);
-                            if (lane == 0) norm_red[egroup][u][q] = sq;
-                        }
-                        if (egroup == 0) asm volatile("bar.sync 3, 128;" ::: "memory");
-                        else asm volatile("bar.sync 4, 128;" ::: "memory");
-                        if (q == 0 && lane < EB && cc0 + 2 * lane < c_hi && tok0 + cc0 + 2 * lane < a.T)
-                            a.norm_ssq[(long)(tok0 + cc0 + 2 * lane) * a.norm_p + tile / tok_tiles] =
-                                ((norm_red[egroup][lane][0] + norm_red[egroup][lane][1]) + norm_red[egroup][lane][2]) +
-                                norm_red[egroup][lane][3];
-                        if (egroup == 0) asm volatile("bar.sync 3, 128;" ::: "memory");
-                        else asm volatile("bar.sync 4, 128;" ::: "memory");
-                    }
+                    const float sq = warp_sum(xn * xn);
+                    if (lane == 0) norm_red[egroup][q] = sq;
+                    if (egroup == 0) asm volatile("bar.sync 3, 128;" ::: "memory");
+                    else asm volatile("bar.sync 4, 128;" ::: "memory");
+                    if (q == 0 && lane == 0)
+                        a.norm_ssq[(long)tok * a.norm_p + tile / tok_tiles] =
+                            ((norm_red[egroup][0] + norm_red[egroup][1]) + norm_red[egroup][2]) + norm_red[egroup][3];
+                    if (egroup == 0) asm volatile("bar.sync 3, 128;" ::: "memory");
+                    else asm volatile("bar.sync 4, 128;" ::: "memory");
                 }
             }
-        } else if constexpr (!C::SPLIT) {
+        } else {
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++local) {
             const int row0 = (tile / tok_tiles) * TC_BM, tok0 = (tile % tok_tiles) * BN;
             const int ab = local & 1;
@@ -748,7 +671,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             if (lane == 0) mbar_arrive(acc_empty0 + 8 * ab);
         }
         }
-        if (a.tma_store && !split && warp == 2 && lane == 0) tma_store_wait_read();
+        if (!C::SPLIT && a.tma_store && warp == 2 && lane == 0) tma_store_wait_read();
         __syncwarp();
     }
 
@@ -758,7 +681,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             cluster_wait();
             cluster_sync_arrive_wait();
         }
-    } else if (split) {
+    } else if constexpr (C::SPLIT) {
         // every thread of every rank passes two cluster barriers: after the partials are written
         // (rank 0's epilogue passes the first one inside its loop) and after they are read
         if (!first_cluster_barrier_done) cluster_sync_arrive_wait();
@@ -1090,7 +1013,7 @@ static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const CUtenso
     return e == cudaSuccess ? launch_status() : (int)e;
 }
 
-// Launches that split K, tiles of at most 32 tokens: the number of stages by blocks and K blocks (see TcCfg).
+// Launches that split K, tiles of at most 64 tokens: the number of stages by tile, blocks and K blocks (see TcCfg).
 template <int BN, int MODE>
 static int launch_split(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& my, const TcArgs& a, cudaStream_t s) {
     // stages and the memory the sums arrive in: two blocks an SM
