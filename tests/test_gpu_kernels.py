@@ -326,6 +326,25 @@ def test_float32_products_of_more_tokens_than_one_call_makes_ready(K):
         assert torch.equal(part, out[at:at + 64]), at
 
 
+def test_float32_products_without_room_for_the_tokens_parts(K, monkeypatch):
+    """The product takes scratch memory from 65 tokens on and needs none: where it gets none the bits are the same."""
+    x, w = rnd((300, 520), torch.float32, seed=45).to(DEV), rnd((130, 520), torch.float32, seed=46).to(DEV)
+    want, out = torch.empty(300, 130, device=DEV), torch.empty(300, 130, device=DEV)
+    K.gemm_generic(x, w, want)
+    real, refused = torch.empty, []
+
+    def empty(*size, **how):
+        if how.get("dtype") == torch.uint8:
+            refused.append(size)
+            raise torch.OutOfMemoryError("no room")
+        return real(*size, **how)
+
+    monkeypatch.setattr(torch, "empty", empty)
+    K.gemm_generic(x, w, out)
+    monkeypatch.undo()
+    assert refused and torch.equal(out, want)
+
+
 def test_gemm_generic_strided_rows_and_true_float32(K):
     """Rows of a wider buffer; and float32 products are not rounded to a shorter mantissa."""
     buf = rnd((10, 100), torch.float32, seed=9).to(DEV)

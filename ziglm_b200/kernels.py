@@ -1139,7 +1139,10 @@ def gemm_generic(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Opti
         scratch, size = None, 0
         if M > 64:
             size = int(_fn("gemm_generic", "zlm_gemm_float_scratch")(M, K))
-            scratch = torch.empty(size, dtype=torch.uint8, device=x.device)
+            try:
+                scratch = torch.empty(size, dtype=torch.uint8, device=x.device)
+            except torch.OutOfMemoryError:          # at most 128 MB: without it the same bits, 64 tokens at a time
+                size = 0
         _check(_fn("gemm_generic", "zlm_gemm_float")(
             x.data_ptr(), w.data_ptr(), _ptr(bias), code(bias.dtype) if bias is not None else F32, out.data_ptr(),
             int(accumulate), M, N, K, x.stride(0) if M > 1 else K, w.stride(0) if N > 1 else K,
