@@ -26,7 +26,8 @@ def rnd(shape, dtype, scale=1.0, seed=0):
 @pytest.fixture(scope="module")
 def K():
     from ziglm_b200 import kernels
-    return kernels
+    yield kernels
+    assert all(code == 0 for code in kernels.wait_errors().values())     # no bounded wait ran out in any test
 
 
 # ------------------------------------------------------------------ elementwise
@@ -118,14 +119,14 @@ def test_gemm_generic(K, xd, wd, yd, M, N, K_):
 @pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("N,K_", [(130, 64), (33, 1000), (4100, 520), (31, 4), (256, 4096), (16500, 200), (20001, 36)])
 def test_few_tokens_in_float32_take_the_streaming_kernel_and_keep_the_order_of_the_sums(K, M, N, K_):
-    """Float operands with at most 32 tokens run a kernel that streams 16 to 128 weight rows a block.  It adds every
-    output's products in the order that K alone sets, so the rows of a step of few tokens equal, bit for bit, the same
-    rows computed inside a step of many tokens."""
+    """Float operands with at most 16 and at most 32 tokens run tiles of 16 and 32.  They add every output's products in the
+    order that K alone sets, so the rows of a step of few tokens equal, bit for bit, the same rows computed inside a step of
+    many tokens."""
     x, w, b = rnd((M, K_), torch.float32, seed=5), rnd((N, K_), torch.float32, seed=6), rnd((N,), torch.float32, seed=7)
     out = torch.full((M, N), 9.0, device=DEV)
     K.gemm_generic(x.to(DEV), w.to(DEV), out, bias=b.to(DEV))
     assert torch.allclose(out.cpu(), P.linear(x, w, b), atol=1e-5 * max(1.0, K_ ** 0.5), rtol=1e-5)
-    # the same rows as the first M of 70 tokens (the tiled kernel)
+    # the same rows as the first M of 70 tokens (tiles of 128, the tokens' parts from memory)
     many = torch.cat([x, rnd((70 - M, K_), torch.float32, seed=8)])
     out_many = torch.empty(70, N, device=DEV)
     K.gemm_generic(many.to(DEV), w.to(DEV), out_many, bias=b.to(DEV))
@@ -142,10 +143,9 @@ def test_few_tokens_in_float32_take_the_streaming_kernel_and_keep_the_order_of_t
 
 @pytest.mark.parametrize("M,N,K_", [(97, 130, 64), (200, 257, 1000), (128, 128, 16), (300, 31, 4), (129, 640, 520)])
 def test_many_tokens_in_float32_take_the_large_tiles_and_keep_the_order_of_the_sums(K, M, N, K_):
-    """Float operands with many tokens run tiles of 64 x 64 or 128 x 128.  The order of an output's additions is set by K
-    alone: rows computed there equal, bit for bit, the same rows computed 70 at a time and 8 at a time (the streaming
-    kernel); so do rows that accumulate and rows of wider buffers; unaligned rows take the kernel of any operands and give
-    the same bits."""
+    """Float operands with many tokens run tiles of 128 x 128.  The order of an output's additions is set by K alone: rows
+    computed there equal, bit for bit, the same rows computed 70 at a time and 8 at a time (tiles of 16 tokens); so do rows
+    that accumulate and rows of wider buffers; unaligned rows are copied four bytes at a time and give the same bits."""
     x, w, b = rnd((M, K_), torch.float32, seed=15), rnd((N, K_), torch.float32, seed=16), rnd((N,), torch.float32, seed=17)
     out = torch.full((M, N), 9.0, device=DEV)
     K.gemm_generic(x.to(DEV), w.to(DEV), out, bias=b.to(DEV))
@@ -162,7 +162,7 @@ def test_many_tokens_in_float32_take_the_large_tiles_and_keep_the_order_of_the_s
     plain = torch.empty(M, N, device=DEV)
     K.gemm_generic(x.to(DEV), w.to(DEV), plain)
     assert torch.equal(acc[:, :N], base[:, :N] + plain) and torch.equal(acc[:, N:], base[:, N:])
-    # rows that start on no 16-byte boundary: the small tiles, the same bits
+    # rows that start on no 16-byte boundary: the same bits
     odd_x = torch.zeros(M, K_ + 8, device=DEV)
     odd_x[:, 1:1 + K_] = x.to(DEV)
     other = torch.empty(M, N, device=DEV)
@@ -170,22 +170,22 @@ def test_many_tokens_in_float32_take_the_large_tiles_and_keep_the_order_of_the_s
     assert torch.equal(other, plain)
 
 
-# fewer blocks of 64 rows than SMs (16 rows; 32 rows: 4096), about as many, two to four times as many (128 rows, few tokens)
+# one to eight segments, whole and ragged, one to 235 tiles of weight rows
 @pytest.mark.parametrize("N,K_", [(65, 1024), (130, 1028), (64, 2052), (3, 8196), (200, 14336), (4097, 516), (9601, 132),
                                   (9602, 1028), (30001, 36)])
 def test_float32_sums_in_segments_of_k(K, N, K_):
-    """Float operands: the K range is cut into at most eight segments whose sums are added in order, by the blocks of a
-    cluster where rows start on 16-byte boundaries and by one block where they do not.  Every number of tokens (the
-    kernels' tiles take up to 1, 2, 4, 8, 16, 32, 64, then 64 or 128 at a time) gives the same bits, and the sums lie
-    within the bound of their own order of additions: the products of a segment one after another, then the segments."""
-    n = min(8, -(-K_ // 1024))
-    seg = -(-(-(-K_ // n)) // 128) * 128
+    """Float operands: the K range is cut into one, two, four or eight segments whose sums are added pairwise, by one block
+    or by the blocks of a cluster.  Every number of tokens (tiles of 16, 32, 64 and 128) gives the same bits, and the sums
+    lie within the bound of their own order of additions: 64 k in the tensor core, which cuts instead of rounding (16 parts
+    in 2^24 cover its four instructions), their sums one after another, then the segments' and the bias."""
+    n = 1 if K_ <= 256 else 2 if K_ <= 512 else 4 if K_ <= 1024 else 8
+    seg = -(-(-(-K_ // n)) // 64) * 64
     x, w = rnd((200, K_), torch.float32, seed=21).to(DEV), rnd((N, K_), torch.float32, seed=22).to(DEV)
     b = rnd((N,), torch.float32, seed=23).to(DEV)
     out = torch.full((200, N), 9.0, device=DEV)
     K.gemm_generic(x, w, out, bias=b)
     want = x.double() @ w.double().t() + b.double()
-    bound = (min(seg, K_) + n + 1) * 2.0 ** -24 * (x.abs().double() @ w.abs().double().t() + b.abs().double())
+    bound = (16 + -(-min(seg, K_) // 64) + 3 + 2) * 2.0 ** -24 * (x.abs().double() @ w.abs().double().t() + b.abs().double())
     assert ((out.double() - want).abs() <= bound).all()
     for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129, 192):
         part = torch.full((M, N), 9.0, device=DEV)
@@ -231,6 +231,35 @@ def test_float32_products_at_the_ends_of_the_range(K, M):
     out = torch.empty(M, N, device=DEV)
     K.gemm_generic(x, one, out)
     assert torch.equal(out, x[:, :N])
+    K.gemm_generic(torch.eye(M, K_, device=DEV), w, out)
+    assert torch.equal(out, w[:, :M].t())
+
+
+@pytest.mark.parametrize("M", [1, 16, 32, 64, 200])
+@pytest.mark.parametrize("K_,offset", [(4096, 0), (14336, 0), (4096, 1)])
+def test_float32_products_are_nearer_to_64_bits_than_one_fmaf_a_product(K, M, K_, offset):
+    """Every tile's width, rows on and off 16-byte boundaries.  Seen: 1.0e-7 over 4,096 and 1.3e-7 over 14,336 (one fmaf a
+    product: 5.7e-7, 7.6e-7); without a1 b1 or one of the smallest products kept it is 2e-6 and more."""
+    N = 256
+    x = rnd((M, K_ + offset), torch.float32, seed=71).to(DEV)[:, offset:]
+    w = rnd((N, K_), torch.float32, seed=72).to(DEV)
+    out = torch.empty(M, N, device=DEV)
+    K.gemm_generic(x, w, out)
+    want = x.double() @ w.double().t()
+    assert (out.double() - want).norm() / want.norm() <= 2e-7
+
+
+@pytest.mark.parametrize("M", [1, 17, 64, 65])
+@pytest.mark.parametrize("K_", [1, 4])
+def test_float32_products_of_a_single_k_keep_the_six_largest_products_of_parts(K, M, K_):
+    """a = 1 + 2^-8 - 2^-17 is 1 + 1 2^-8 - 1/2 2^-16 in parts: of a^2 the kernel leaves out 2 a1 a2 = -2^-24 and a2^2 = 2^-34,
+    the most that any pair loses (1.0 parts in 2^24), and every product that it keeps is at least 2^-17."""
+    a = 1.0 + 2.0 ** -8 - 2.0 ** -17
+    x, w = torch.zeros(M, K_, device=DEV), torch.zeros(130, K_, device=DEV)
+    x[:, -1], w[:, -1] = a, a
+    out = torch.empty(M, 130, device=DEV)
+    K.gemm_generic(x, w, out)
+    assert ((out.double() - a * a).abs() <= 2 * 2.0 ** -24 * a * a).all()
 
 
 @pytest.mark.parametrize("M", [1, 17, 64, 200])
