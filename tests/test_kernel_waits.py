@@ -7,7 +7,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "ziglm_b200", "csrc")
-FILES = ["attention_fmha.cu", "attention_tc.cu", "gemm_tc.cu", "tc_common.cuh"]
+FILES = ["attention_fmha.cu", "attention_tc.cu", "gemm_generic.cu", "gemm_tc.cu", "tc_common.cuh"]
 ONE_LANE = re.compile(r"\blane == 0\b|\bthreadIdx\.x == 0\b")
 
 
