@@ -996,7 +996,9 @@ attn_decode_flat_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                     v.x += __shfl_xor_sync(0xffffffffu, v.x, o); v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
                     v.z += __shfl_xor_sync(0xffffffffu, v.z, o); v.w += __shfl_xor_sync(0xffffffffu, v.w, o);
                 }
-                if (u == 0 && f < quads) store_quad(v, den, grow, f, orow);
+                // an output a lane: one quotient's code (four by the first lane: one sequence at the 1B shape 4 us a step longer)
+                const float sum = u == 0 ? v.x : u == 1 ? v.y : u == 2 ? v.z : v.w;
+                if (u < 4 && f < quads) orow[4 * f + u] = __float2bfloat16_rn(sum / den * gate_factor(grow, 4 * f + u));
             }
             cluster_sync_arrive_wait();            // the others may still read this block's piece
             break;
