@@ -1737,7 +1737,8 @@ def attention(step, qkv: torch.Tensor, out: torch.Tensor, n_heads: int, n_kv: in
             room = _flat_room(step, n_heads, n_kv, head_dim) if keep_first == 0 and head_gate is None else None
             # a block of the flat kernel merges a sequence's pieces alone: with many pieces (few sequences and key/value
             # heads) the second kernel of the other, which merges rows side by side, is faster (43 against 50 us at eight
-            # sequences of 4,096 tokens on one key/value head)
+            # sequences of 4,096 tokens on one key/value head; measured before steps of few items took clusters, whose blocks
+            # merge together, and not again since)
             if room is not None and step.n_tokens * n_kv * FLAT_PIECES >= room[0] and attention_decode_flat(
                     qkv, out, n_heads, n_kv, head_dim, scale, window, step.positions, step.seq_of_token, io.block_table,
                     io.k_pages, io.v_pages, io.page_size, *room, softcap=softcap, gate=gate, sinks=sinks, slopes=slopes):
